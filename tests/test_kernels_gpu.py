@@ -286,6 +286,27 @@ def test_paged_attention(ops, dtype, nq, nkv, hd, page, window):
         assert float(p[3]) > 0.9
 
 
+@pytest.mark.parametrize("m,n,k", [(17, 64, 4), (17, 2561, 20), (33, 4801, 36), (100, 2560, 64), (65, 9473, 16), (509, 2560, 40),
+                                   (64, 12161, 68), (513, 130, 1028)])
+def test_float32_tiles_of_every_size_give_the_bits_of_the_tile_kernel(ops, m, n, k, monkeypatch):
+    """Each tile shape of the products of more than 16 float32 rows (one row or column behind whole tiles, depths that
+    fill no step, a single step, more steps than are in flight), strided operands, stored and added."""
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k + 4, device=DEV)[:, :k]
+    w = torch.randn(n, k, device=DEV)
+    outs = []
+    for tiles in (True, False):
+        monkeypatch.setattr(ops, "linear_skinny", tiles)
+        out = torch.full((m, n + 3), 7.0, device=DEV)
+        ops.linear(a, w, out[:, :n])
+        acc = torch.full((m, n), 0.25, device=DEV)
+        ops.linear(a, w, acc, accumulate=True)
+        outs.append((out, acc))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    ref = a.double() @ w.double().T
+    assert float((outs[0][0][:, :n] - ref).abs().max()) <= k * 2.0 ** -23 * float(a.abs().max() * w.abs().max()) * math.sqrt(k)
+
+
 @pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("window", [None, 300])
 @pytest.mark.parametrize("nq,nkv,hd", [(6, 2, 48), (8, 1, 64), (4, 4, 128), (10, 2, 256)])

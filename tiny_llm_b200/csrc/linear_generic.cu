@@ -1,10 +1,10 @@
 // C[M,N] = A[M,K] . W[N,K]^T on the CUDA cores with 32-bit accumulation (FFMA only, no tensor-core
 // mode): the product of the true 32-bit path, and the fallback of the bfloat16 path for sizes the
 // tensor-core kernels refuse.  Any M, N, K.  Every output element is ONE chain of fmaf over k in
-// ascending order starting from zero, whatever M is and whichever of the two kernels below computes it,
+// ascending order starting from zero, whatever M is and whichever of the kernels below computes it,
 // so a row's result does not depend on its batch, to the bit.
 //   linear_generic_kernel: 64 x 64 tiles, 4 x 4 outputs per thread (any sizes and both dtypes);
-//   linear_large_kernel: float32, 128 x 128 tiles, 8 x 8 outputs per thread (products of at least 128 x 128);
+//   linear_tiled_kernel: float32, more than 16 rows, rows on 16 bytes: tiles from 16 x 64 to 64 x 192 by the sizes;
 //   linear_skinny_kernel: float32, at most 16 rows (decoded tokens): a CTA takes 8 or 16 weight rows and
 //     streams them through shared memory in chunks of 128 k (cp.async, three stages), one thread per
 //     output element.  With so few rows the 64-row tile left 32 CTAs to stream a matrix that 148 SMs could
@@ -82,96 +82,218 @@ linear_generic_kernel(const T* __restrict__ a, const T* __restrict__ w, void* __
   }
 }
 
-// ---------------------------------------------------------------- many rows: 128 x 128 tiles, 8 x 8 outputs per thread
-// The same chains of fmaf (k ascending from zero for every output element), with an eighth of the shared-memory reads
-// per fmaf of the 64 x 64 kernel: 16-byte global loads of the next 16-wide slice of k into registers while the current
-// one is multiplied, shared memory transposed to [k][row] so that a thread's eight rows (and eight columns) are two
-// 16-byte reads.  Taken for products of at least 128 x 128 whose rows start on 16 bytes; float32 only.
-constexpr int LBM = 128, LBN = 128, LBK = 16, LTHREADS = 256;
+// ---------------------------------------------------------------- more than 16 rows, float32: tiles of fma pairs
+// The same chains of fmaf (k ascending from zero for every output element; fma.rn.f32x2 rounds each half like fmaf).
+// What bounds it: the fma pipe.  A packed fma keeps the pipe busy for two cycles with one issue slot, which leaves the
+// other slot for the operands; a thread's outputs are pairs of neighbouring columns, so that a pair of weights is one
+// half of a 16-byte read and only the row's value has to be doubled in a register.
+// Two producer warps beside the computing ones keep cp.async copies of the next TST steps of TBK values of k in flight
+// (a step of products is shorter than a trip to memory: with one step of look-ahead in registers a CTA alone on an SM
+// took 182 cycles per k for 128 x 128 outputs) and turn each landed step into [k][row] order, from which a computing
+// thread reads four rows or four columns at once, while the step before is multiplied: one barrier per step.
+// Measured on 509 x 2,048 x 2,048 / 509 x 11,264 x 2,048 / 509 x 2,048 x 5,632, us: 128 x 128 tiles of single fmaf with
+// register look-ahead 239 / 697 / 638; these tiles 102 / 457 / 269 (the pipe's own time: 57 / 316 / 158).
+__device__ __forceinline__ uint64_t pack_pair(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack_pair(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// 16 bytes on their way to shared memory; ok = false fills them with zeros, which leave a chain of fmaf as it is
+__device__ __forceinline__ void copy16_async(uint32_t dst, const float* src, bool ok) {
+  const int bytes = ok ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
 
-template <int MODE>
-__global__ void __launch_bounds__(LTHREADS)
-linear_large_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ out,
+constexpr int TBK = 16, TST = 4, TPRODUCERS = 64;
+
+// WM x WN computing warps, each (4 TM) x (8 TN) outputs, a thread TM x TN
+template <int WM, int WN, int TM, int TN>
+struct Tile {
+  static constexpr int M = WM * 4 * TM, N = WN * 8 * TN, COMPUTE = WM * WN * 32, THREADS = COMPUTE + TPRODUCERS;
+  static constexpr int PM = M + 4, PN = N + 4;                 // pitches of the [k][row] tiles
+  static constexpr int RAW = (M + N) * TBK;                    // floats of a landed step: rows of A, then rows of W
+  static constexpr int SMEM = (TST * RAW + 2 * TBK * (PM + PN)) * (int)sizeof(float);
+  static constexpr int SMEM_ALONE = 120000;                    // more than half of an SM's: one CTA per SM
+};
+
+template <int WM, int WN, int TM, int TN, int MODE>
+__global__ void __launch_bounds__((Tile<WM, WN, TM, TN>::THREADS), (TM * TN > 64 ? 1 : 2))
+linear_tiled_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ out,
                     int m, int n, int k, int lda, int ldo) {
-  __shared__ __align__(16) float as[2][LBK][LBM + 4];
-  __shared__ __align__(16) float ws[2][LBK][LBN + 4];
+  using C = Tile<WM, WN, TM, TN>;
+  constexpr int PM = C::PM, PN = C::PN, QK = TBK / 4;
+  constexpr int LA = C::M * QK / TPRODUCERS, LW = C::N * QK / TPRODUCERS;   // 16-byte copies per producer and step
+  static_assert(LA * TPRODUCERS == C::M * QK && LW * TPRODUCERS == C::N * QK, "whole copies per producer");
+  extern __shared__ __align__(16) float tile_smem[];
+  float* raw = tile_smem;
+  float* as = tile_smem + TST * C::RAW;       // [2][TBK][PM]
+  float* ws = as + 2 * TBK * PM;              // [2][TBK][PN]
   pdl_trigger();
-  pdl_wait();
   const int tid = threadIdx.x;
-  const int tx = tid % 16, ty = tid / 16;          // this thread's columns tx * 4 + {0..3} and 64 + tx * 4 + {0..3}; rows likewise
-  const int m0 = blockIdx.y * LBM, n0 = blockIdx.x * LBN;
-  // loader: thread -> (row lr of the tile, k quad lq); two rows per operand (lr and lr + 64)
-  const int lr = tid / 4, lq = (tid % 4) * 4;
-  float acc[8][8];
+  const int m0 = blockIdx.x * C::M, n0 = blockIdx.y * C::N;
+  const int steps = (k + TBK - 1) / TBK;
+
+  if (tid >= C::COMPUTE) {
+    // ---------------- producers
+    const int pt = tid - C::COMPUTE;
+    const uint32_t raw_u = (uint32_t)__cvta_generic_to_shared(raw);
+    auto copy_w = [&](int st) {
+      if (st >= steps) return;
+      const uint32_t d = raw_u + (uint32_t)((st % TST) * C::RAW + C::M * TBK) * 4u;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < LW; ++i) {
+        const int idx = pt + i * TPRODUCERS, r = n0 + idx / QK, kk = st * TBK + (idx % QK) * 4;   // k is a multiple of 4
+        const bool ok = r < n && kk < k;
+        copy16_async(d + idx * 16, ok ? w + (size_t)r * k + kk : w, ok);
+      }
+    };
+    auto copy_a = [&](int st) {
+      if (st >= steps) return;
+      const uint32_t d = raw_u + (uint32_t)((st % TST) * C::RAW) * 4u;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  float4 ra[2], rw[2];
-  auto fetch = [&](int k0) {
+      for (int i = 0; i < LA; ++i) {
+        const int idx = pt + i * TPRODUCERS, r = m0 + idx / QK, kk = st * TBK + (idx % QK) * 4;
+        const bool ok = r < m && kk < k;
+        copy16_async(d + idx * 16, ok ? a + (size_t)r * lda + kk : a, ok);
+      }
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    for (int st = 0; st < TST; ++st) copy_w(st);   // the weights depend on no earlier kernel
+    pdl_wait();
+    for (int st = 0; st < TST; ++st) { copy_a(st); commit(); }
+    for (int st = 0; st < steps; ++st) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(TST - 1) : "memory");
+      // a producer turns what it copied itself, so its own landed groups are all it has to wait for
+      const float4* rs = reinterpret_cast<const float4*>(raw + (st % TST) * C::RAW);
+      float* ad = as + (st & 1) * TBK * PM;
+      float* wd = ws + (st & 1) * TBK * PN;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int gm = m0 + lr + 64 * h, gn = n0 + lr + 64 * h, kk = k0 + lq;
-      ra[h] = (gm < m && kk < k) ? *reinterpret_cast<const float4*>(a + (size_t)gm * lda + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
-      rw[h] = (gn < n && kk < k) ? *reinterpret_cast<const float4*>(w + (size_t)gn * k + kk) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < LA; ++i) {
+        const int idx = pt + i * TPRODUCERS, r = idx / QK, q = (idx % QK) * 4;
+        const float4 v = rs[idx];
+        ad[q * PM + r] = v.x; ad[(q + 1) * PM + r] = v.y; ad[(q + 2) * PM + r] = v.z; ad[(q + 3) * PM + r] = v.w;
+      }
+#pragma unroll
+      for (int i = 0; i < LW; ++i) {
+        const int idx = pt + i * TPRODUCERS, r = idx / QK, q = (idx % QK) * 4;
+        const float4 v = rs[C::M * QK + idx];
+        wd[q * PN + r] = v.x; wd[(q + 1) * PN + r] = v.y; wd[(q + 2) * PN + r] = v.z; wd[(q + 3) * PN + r] = v.w;
+      }
+      copy_w(st + TST);
+      copy_a(st + TST);
+      commit();
+      __syncthreads();   // step st can be read; everyone has left step st - 1, whose place step st + 1 takes
     }
-  };
-  auto stash = [&](int buf) {
+    return;
+  }
+
+  // ---------------- computing warps
+  pdl_wait();
+  const int warp = tid >> 5, lane = tid & 31;
+  const int ar0 = (warp / WN) * 4 * TM + (lane / 8) * 4;   // this thread's rows: ar0 + 16 i + {0..3}
+  const int bc0 = (warp % WN) * 8 * TN + (lane % 8) * 4;   // ... and columns: bc0 + 32 j + {0..3}
+  uint64_t acc[TM][TN / 2];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int r = lr + 64 * h;
-      as[buf][lq + 0][r] = ra[h].x; as[buf][lq + 1][r] = ra[h].y; as[buf][lq + 2][r] = ra[h].z; as[buf][lq + 3][r] = ra[h].w;
-      ws[buf][lq + 0][r] = rw[h].x; ws[buf][lq + 1][r] = rw[h].y; ws[buf][lq + 2][r] = rw[h].z; ws[buf][lq + 3][r] = rw[h].w;
-    }
-  };
-  fetch(0);
-  stash(0);
-  __syncthreads();
-  int buf = 0;
-  for (int k0 = 0; k0 < k; k0 += LBK) {
-    const bool more = k0 + LBK < k;
-    if (more) fetch(k0 + LBK);
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int p = 0; p < LBK; ++p) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&as[buf][p][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&as[buf][p][64 + ty * 4]);
-      const float4 w0 = *reinterpret_cast<const float4*>(&ws[buf][p][tx * 4]);
-      const float4 w1 = *reinterpret_cast<const float4*>(&ws[buf][p][64 + tx * 4]);
-      const float ar[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float wr[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
+#pragma unroll 1
+  for (int st = 0; st < steps; ++st) {
+    __syncthreads();
+    const float* ab = as + (st & 1) * TBK * PM + ar0;
+    const float* wb = ws + (st & 1) * TBK * PN + bc0;
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+    for (int p = 0; p < TBK; ++p) {
+      float4 a4[TM / 4];
+      ulonglong2 w4[TN / 4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
-    }
-    if (more) {
-      stash(buf ^ 1);
-      __syncthreads();
-      buf ^= 1;
+      for (int i = 0; i < TM / 4; ++i) a4[i] = *reinterpret_cast<const float4*>(ab + p * PM + 16 * i);
+#pragma unroll
+      for (int j = 0; j < TN / 4; ++j) w4[j] = *reinterpret_cast<const ulonglong2*>(wb + p * PN + 32 * j);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const float av = (i & 3) == 0 ? a4[i / 4].x : (i & 3) == 1 ? a4[i / 4].y : (i & 3) == 2 ? a4[i / 4].z : a4[i / 4].w;
+        const uint64_t aa = pack_pair(av, av);
+#pragma unroll
+        for (int j = 0; j < TN / 4; ++j) {
+          acc[i][2 * j] = fma_pair(aa, w4[j].x, acc[i][2 * j]);
+          acc[i][2 * j + 1] = fma_pair(aa, w4[j].y, acc[i][2 * j + 1]);
+        }
+      }
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
+  for (int i = 0; i < TM; ++i) {
+    const int gm = m0 + ar0 + 16 * (i / 4) + (i & 3);
     if (gm >= m) continue;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int gn = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
+    for (int j = 0; j < TN; ++j) {
+      const int gn = n0 + bc0 + 32 * (j / 4) + (j & 3);
       if (gn >= n) continue;
+      float lo, hi;
+      unpack_pair(acc[i][j / 2], lo, hi);
+      const float v = (j & 1) ? hi : lo;
       const size_t o = (size_t)gm * ldo + gn;
-      if (MODE == OUT_ACC) out[o] += acc[i][j];
-      else out[o] = acc[i][j];
+      if (MODE == OUT_ACC) out[o] += v;
+      else out[o] = v;
     }
   }
 }
 
-static int launch_large(const float* a, const float* w, float* out, int m, int n, int k, int lda, int ldo, int mode, cudaStream_t s) {
-  dim3 grid((n + LBN - 1) / LBN, (m + LBM - 1) / LBM);
-  if (mode == OUT_ACC)
-    TLLM_LAUNCH("linear_large", linear_large_kernel<OUT_ACC>, grid, LTHREADS, 0, s, a, w, out, m, n, k, lda, ldo);
-  else
-    TLLM_LAUNCH("linear_large", linear_large_kernel<OUT_F32>, grid, LTHREADS, 0, s, a, w, out, m, n, k, lda, ldo);
+template <int WM, int WN, int TM, int TN, int MODE>
+static int launch_tile_mode(const float* a, const float* w, float* out, int m, int n, int k, int lda, int ldo, int sms, cudaStream_t s) {
+  using C = Tile<WM, WN, TM, TN>;
+  auto kern = linear_tiled_kernel<WM, WN, TM, TN, MODE>;
+  constexpr int MOST = C::SMEM > C::SMEM_ALONE ? C::SMEM : C::SMEM_ALONE;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
+    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "linear_tiled: cannot reserve %d bytes of shared memory: %s", MOST, cudaGetErrorString(e));
+    configured = true;
+  }
+  dim3 grid((m + C::M - 1) / C::M, (n + C::N - 1) / C::N);
+  // As many CTAs as SMs or fewer: one per SM.  Two that may share an SM do so while others idle (128 CTAs of 64 x 128
+  // took 155 us instead of 102).
+  const int smem = (long long)grid.x * grid.y <= sms ? MOST : C::SMEM;
+  TLLM_LAUNCH("linear_tiled", kern, grid, C::THREADS, smem, s, a, w, out, m, n, k, lda, ldo);
   return TLLM_OK;
+}
+
+template <int WM, int WN, int TM, int TN>
+static int launch_tile(const float* a, const float* w, float* out, int m, int n, int k, int lda, int ldo, int mode, int sms, cudaStream_t s) {
+  if (mode == OUT_ACC) return launch_tile_mode<WM, WN, TM, TN, OUT_ACC>(a, w, out, m, n, k, lda, ldo, sms, s);
+  return launch_tile_mode<WM, WN, TM, TN, OUT_F32>(a, w, out, m, n, k, lda, ldo, sms, s);
+}
+
+// Which tile: the one whose rounds over the SMs cost least, with the measured cycles per k of a tile alone on an SM.
+// (m x n x k, us, chosen against the other tiles: 509 x 2,560 x 2,048 64 x 192 147 / 64 x 128 193; 200 x 2,560 64 x 128
+// 100 / 64 x 64 128; 100 x 2,560 64 x 64 73 / 64 x 128 100; 100 x 2,048 x 5,632 32 x 64 152 / 64 x 64 193;
+// 40 x 2,560 16 x 64 39 / 32 x 64 57; 40 x 11,264 64 x 128 100 / 16 x 64 135.)
+static int launch_tiled(const float* a, const float* w, float* out, int m, int n, int k, int lda, int ldo, int mode, cudaStream_t s) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+    TLLM_FAIL(TLLM_ERR_CUDA, "linear: cannot read the number of SMs");
+  static const struct { int m, n, cycles; } kinds[] = {{64, 128, 95}, {64, 192, 137}, {64, 64, 70}, {32, 64, 54}, {16, 64, 37}};
+  int best = 0;
+  long long best_cost = -1;
+  for (int i = 0; i < 5; ++i) {
+    const long long ctas = (long long)((m + kinds[i].m - 1) / kinds[i].m) * ((n + kinds[i].n - 1) / kinds[i].n);
+    const long long cost = (ctas + sms - 1) / sms * kinds[i].cycles;
+    if (best_cost < 0 || cost < best_cost) { best = i; best_cost = cost; }
+  }
+  switch (best) {
+    case 0: return launch_tile<2, 2, 8, 8>(a, w, out, m, n, k, lda, ldo, mode, sms, s);
+    case 1: return launch_tile<2, 2, 8, 12>(a, w, out, m, n, k, lda, ldo, mode, sms, s);
+    case 2: return launch_tile<2, 2, 8, 4>(a, w, out, m, n, k, lda, ldo, mode, sms, s);
+    case 3: return launch_tile<2, 2, 4, 4>(a, w, out, m, n, k, lda, ldo, mode, sms, s);
+    default: return launch_tile<1, 2, 4, 4>(a, w, out, m, n, k, lda, ldo, mode, sms, s);
+  }
 }
 
 // ---------------------------------------------------------------- at most 16 rows, float32
@@ -302,9 +424,9 @@ extern "C" int tllm_linear_generic(const void* a, const void* w, void* out, int 
     if (m <= 8) return tllm::launch_skinny<8>(af, wf, of, m, n, k, lda, ldo, mode, s);
     return tllm::launch_skinny<16>(af, wf, of, m, n, k, lda, ldo, mode, s);
   }
-  if (dtype == TLLM_F32 && skinny != 0 && m >= 128 && n >= 128 && k % 4 == 0 && lda % 4 == 0 && ((uintptr_t)a % 16) == 0 &&
-      ((uintptr_t)w % 16) == 0 && (m + tllm::LBM - 1) / tllm::LBM <= 65535)
-    return tllm::launch_large((const float*)a, (const float*)w, (float*)out, m, n, k, lda, ldo, mode, (cudaStream_t)stream);
+  if (dtype == TLLM_F32 && skinny != 0 && m > 16 && k % 4 == 0 && lda % 4 == 0 && ((uintptr_t)a % 16) == 0 && ((uintptr_t)w % 16) == 0 &&
+      n <= 64 * 65535 && (mode == tllm::OUT_SAME || mode == tllm::OUT_F32 || mode == tllm::OUT_ACC))
+    return tllm::launch_tiled((const float*)a, (const float*)w, (float*)out, m, n, k, lda, ldo, mode, (cudaStream_t)stream);
   if (dtype == TLLM_F32) return tllm::launch<float>(a, w, out, m, n, k, lda, ldo, mode, (cudaStream_t)stream);
   if (dtype == TLLM_BF16) return tllm::launch<__nv_bfloat16>(a, w, out, m, n, k, lda, ldo, mode, (cudaStream_t)stream);
   TLLM_FAIL(TLLM_ERR_ARG, "linear: unknown dtype code %d", dtype);
