@@ -759,3 +759,31 @@ def test_sample_top_k_keeps_exactly_k_with_ties(ops):
                    torch.tensor([c], dtype=torch.int64, device=DEV), out)
         draws.add(int(out[0]))
     assert draws == {5, 9, 50}
+
+
+@pytest.mark.parametrize("vocab", [1, 331, 1024, 1025, 8192, 8193, 16385, 32000, 32768])
+def test_sample_in_registers_draws_what_the_passes_over_memory_draw(ops, vocab):
+    """Rows of up to 32,768 logits are kept in registers, longer ones are walked in memory.  A row filled up to 33,000
+    with minus infinity takes the second way and must give the same id: smooth rows, rows of many equal values, one
+    value throughout, rows with dropped ids, for every kind of limit (none, one, few, more values than are ranked, more
+    than one per thread, all) and mass."""
+    g = torch.Generator().manual_seed(vocab)
+    options = [(t, k, p) for t in (0.7, 1.0) for k in (0, 1, 2, 50, 300, 1024, 1025, vocab) for p in (0.0, 0.1, 0.5, 0.95, 1.0)]
+    kinds = [lambda: torch.randn(vocab, generator=g) * 3, lambda: torch.randint(-4, 5, (vocab,), generator=g).float(),
+             lambda: torch.full((vocab,), 1.5),
+             lambda: torch.where(torch.rand(vocab, generator=g) < 0.7, torch.tensor(-math.inf), torch.randn(vocab, generator=g))]
+    rows = torch.stack([kinds[i % 4]() for i in range(len(options) * 4)])
+    rows[3::4, 0] = 0.25      # not every id dropped
+    options = [o for o in options for _ in range(4)]
+    n = len(options)
+    long = torch.full((n, 33000), -math.inf)
+    long[:, :vocab] = rows
+    temps, ks, ps = (torch.tensor([o[j] for o in options]) for j in range(3))
+    seeds, counters = torch.arange(n, dtype=torch.int64) * 31 + 5, torch.arange(n, dtype=torch.int64) % 3
+    got = []
+    for logits in (rows, long):
+        out = torch.empty(n, dtype=torch.int32, device=DEV)
+        ops.sample(logits.to(DEV), torch.empty(logits.numel(), device=DEV), temps.to(DEV), ks.to(torch.int32).to(DEV),
+                   ps.to(DEV), seeds.to(DEV), counters.to(DEV), out)
+        got.append(out.cpu().tolist())
+    assert got[0] == got[1]

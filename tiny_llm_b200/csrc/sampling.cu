@@ -199,28 +199,10 @@ __device__ __forceinline__ float uniform_from(unsigned long long seed, unsigned 
   return (float)(z >> 40) * (1.0f / 16777216.0f);
 }
 
-__global__ void __launch_bounds__(ST)
-sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int v,
-              const float* __restrict__ temperature, const int* __restrict__ top_k,
-              const float* __restrict__ top_p, const unsigned long long* __restrict__ seeds,
-              const unsigned long long* __restrict__ counters, int* __restrict__ out,
-              const int* __restrict__ status) {
-  __shared__ BlockScratch sc;
+// The choice of one row in passes over its scratch `x` (v floats in global memory), for any length and any limits.
+__device__ __noinline__ void sample_in_memory(const float* __restrict__ row, float* __restrict__ x, int v, float temp, int k,
+                                              float p, float u, int* __restrict__ out, BlockScratch& sc) {
   __shared__ int s_choice, s_last;
-  pdl_trigger();
-  pdl_wait();
-  forward_status(status, out);
-  const int b = blockIdx.x;
-  const float* row = logits + (size_t)b * v;
-  const float temp = temperature[b];
-  if (!(temp > 0.f)) {
-    const int r = block_argmax(row, v, sc);
-    if (threadIdx.x == 0) out[b] = r;
-    return;
-  }
-  float* x = work + (size_t)b * v;
-  const int k = top_k[b];
-  const float p = top_p[b];
 
   // scaled logits and their maximum
   float mx = -CUDART_INF_F;
@@ -290,7 +272,7 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int v,
   }
 
   // multinomial: first token id whose running weight exceeds u * z
-  const float target = uniform_from(seeds[b], counters[b]) * z;
+  const float target = u * z;
   if (threadIdx.x == 0) { s_choice = 0x7fffffff; s_last = -1; }
   __syncthreads();
   float base = 0.f;
@@ -308,7 +290,318 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int v,
     if (s_choice != 0x7fffffff) break;
   }
   __syncthreads();
-  if (threadIdx.x == 0) out[b] = s_choice != 0x7fffffff ? s_choice : s_last;
+  if (threadIdx.x == 0) *out = s_choice != 0x7fffffff ? s_choice : s_last;
+}
+
+__global__ void __launch_bounds__(ST)
+sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int v,
+              const float* __restrict__ temperature, const int* __restrict__ top_k,
+              const float* __restrict__ top_p, const unsigned long long* __restrict__ seeds,
+              const unsigned long long* __restrict__ counters, int* __restrict__ out,
+              const int* __restrict__ status) {
+  __shared__ BlockScratch sc;
+  pdl_trigger();
+  pdl_wait();
+  forward_status(status, out);
+  const int b = blockIdx.x;
+  const float* row = logits + (size_t)b * v;
+  const float temp = temperature[b];
+  if (!(temp > 0.f)) {
+    const int r = block_argmax(row, v, sc);
+    if (threadIdx.x == 0) out[b] = r;
+    return;
+  }
+  sample_in_memory(row, work + (size_t)b * v, v, temp, top_k[b], top_p[b], uniform_from(seeds[b], counters[b]), out + b, sc);
+}
+
+// ---------------------------------------------------------------- rows of at most 32,768 logits: the row in registers
+// The same choice, to the bit, with the row read once: a thread holds the values of its ids chunk * 1,024 + thread.
+// What bounds it is no longer memory but the chain of block-wide agreements and, at one block per row, the code itself
+// (loops unrolled over the registers run once: a first form of this kernel that walked all registers in every phase
+// took 55 us, most of it instruction fetches).  So the registers are walked twice, and what survives is a short list:
+//   top-k   The k-th largest of the threads' maxima bounds the k-th largest value from below (k values are not less);
+//           32 barrier counts find it.  The values from there on, a few more than k, are listed in shared memory and
+//           ranked against one another by value, then id; rank < k stays.
+//   top-p   The sum of the weights below a cut grows with the cut, so the cut is one of the listed weights: they are
+//           sorted and halved (6 sums for 50 weights, where a search over bit patterns takes 31).
+//   draw    The chunks that hold a weight are scanned at once: in every warp, over the warps' sums of a chunk by one
+//           warp per chunk, and over the chunks' sums by every thread that holds a weight.
+// Without a top-k every id has a weight: those rows search the cut over bit patterns, in registers.
+// Lists that do not fit (ties, k > 200 or so) take the passes over memory.
+// Every floating-point sum has the operands and the tree of sample_in_memory (terms left out are zeros there), so the
+// same id is chosen.  us per call, this kernel / the passes over memory: 64 rows
+// of 32,000, k 50, p 0.95 20 / 198; k 200, p 0.9 34 / 200; no top-k, p 0.9 44 / 102; one row 19 / 135; 64 of 8,000 15 / 76.
+constexpr int LISTED = 256;   // values that are ranked against one another
+constexpr int OWN = 4;        // ... and of them per thread
+
+struct RowScratch {
+  BlockScratch block;
+  float sums[2][32];
+  float chunk_warp[32][33];   // [chunk][warp]: sums, then what lies before the warp inside the chunk
+  float chunk_total[32];
+  uint32_t list[LISTED], sorted[LISTED];
+  int ids[LISTED];
+  int listed, overflow, choice, last;
+};
+
+// A sum over the block with one barrier: the tree of block_sum.  Calls alternate between two sets of scratch.
+__device__ __forceinline__ float row_sum(float v, RowScratch& sc, int& turn) {
+  v = warp_sum(v);
+  turn ^= 1;
+  if ((threadIdx.x & 31) == 0) sc.sums[turn][threadIdx.x >> 5] = v;
+  __syncthreads();
+  return warp_sum(sc.sums[turn][threadIdx.x & 31]);
+}
+// Running sum inside the warp, in the order of block_incl_scan_f.
+__device__ __forceinline__ float warp_running_sum(float v) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float n = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += n;
+  }
+  return v;
+}
+// The warps' sums of every chunk become what lies before each warp; the chunks' sums.  All threads; ends with a barrier.
+__device__ __forceinline__ void scan_chunks(RowScratch& sc, int chunks) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __syncthreads();
+  if (warp < chunks) {
+    const float sum = sc.chunk_warp[warp][lane];
+    const float w = warp_running_sum(sum);
+    sc.chunk_warp[warp][lane] = w - sum;
+    if (lane == 31) sc.chunk_total[warp] = w;
+  }
+  __syncthreads();
+}
+
+template <int NV>   // values per thread
+__global__ void __launch_bounds__(ST)
+sample_row_kernel(const float* __restrict__ logits, float* __restrict__ work, int v, const float* __restrict__ temperature,
+                  const int* __restrict__ top_k, const float* __restrict__ top_p,
+                  const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ counters,
+                  int* __restrict__ out, const int* __restrict__ status) {
+  __shared__ RowScratch sc;
+  pdl_trigger();
+  pdl_wait();
+  forward_status(status, out);
+  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const float* row = logits + (size_t)b * v;
+  const float temp = temperature[b];
+  if (!(temp > 0.f)) {
+    const int r = block_argmax(row, v, sc.block);
+    if (tid == 0) out[b] = r;
+    return;
+  }
+  const int k = top_k[b];
+  const float p = top_p[b], u = uniform_from(seeds[b], counters[b]);
+  const uint32_t one = __float_as_uint(1.0f);
+  int turn = 0;
+  if (tid == 0) { sc.listed = 0; sc.overflow = 0; sc.choice = 0x7fffffff; sc.last = -1; }
+  sc.chunk_warp[tid >> 5][tid & 31] = 0.f;
+
+  float x[NV];
+#pragma unroll
+  for (int c = 0; c < NV; ++c) x[c] = c * ST + tid < v ? row[c * ST + tid] : -CUDART_INF_F;
+  float mx = -CUDART_INF_F;
+  uint32_t best = 0;      // the largest key among this thread's ids
+#pragma unroll
+  for (int c = 0; c < NV; ++c) {
+    x[c] = c * ST + tid < v ? x[c] / temp : -CUDART_INF_F;
+    mx = fmaxf(mx, x[c]);
+    if (c * ST + tid < v) best = max(best, ordered_key(x[c]));
+  }
+  mx = block_max_f(mx, sc.block);
+
+  if (k > 0 && k < v) {
+    uint32_t bound = 0;
+    if (k <= LISTED)
+      for (int bit = 31; bit >= 0; --bit) {
+        const uint32_t cand = bound | (1u << bit);
+        if (__syncthreads_count(best >= cand) >= k) bound = cand;
+      }
+    uint32_t mine = 0;      // chunks in which this thread's value reaches the bound
+    if (bound != 0 && best >= bound) {
+#pragma unroll
+      for (int c = 0; c < NV; ++c)
+        if (c * ST + tid < v && ordered_key(x[c]) >= bound) mine |= 1u << c;
+    }
+    const int held = __popc(mine);
+    float own[OWN];
+    int chunk[OWN], at = 0;
+    if (held > 0) {
+      at = atomicAdd(&sc.listed, held);
+      if (held > OWN || at + held > LISTED) sc.overflow = 1;
+    }
+    __syncthreads();
+    const int total = sc.listed;
+    if (bound == 0 || sc.overflow != 0 || total > LISTED) {    // (uniform)
+      sample_in_memory(row, work + (size_t)b * v, v, temp, k, p, u, out + b, sc.block);
+      return;
+    }
+#pragma unroll
+    for (int j = 0; j < OWN; ++j) {
+      own[j] = -CUDART_INF_F;
+      chunk[j] = -1;
+      if (j < held) {
+        chunk[j] = __ffs(mine) - 1;
+        mine &= mine - 1;
+        own[j] = row[chunk[j] * ST + tid] / temp;
+        sc.list[at + j] = ordered_key(own[j]);
+        sc.ids[at + j] = chunk[j] * ST + tid;
+      }
+    }
+    __syncthreads();
+    if (tid < total) {
+      const uint32_t key = sc.list[tid];
+      const int id = sc.ids[tid];
+      int rank = 0;
+      for (int j = 0; j < total; ++j) rank += sc.list[j] > key || (sc.list[j] == key && sc.ids[j] < id);
+      sc.sorted[tid] = rank < k;
+    }
+    __syncthreads();
+    // weights e_i = exp(x_i - max) of the kept tokens, 0 for the dropped ones
+    float z = 0.f;
+#pragma unroll
+    for (int j = 0; j < OWN; ++j) {
+      float e = 0.f;
+      if (j < held && sc.sorted[at + j] != 0 && own[j] != -CUDART_INF_F) e = expf(own[j] - mx);
+      own[j] = e;
+      z += e;
+      if (j < held) sc.list[at + j] = __float_as_uint(e);
+    }
+    z = row_sum(z, sc, turn);
+    if (p < 1.f) {
+      const float budget = (1.f - p) * z;
+      if (tid < total) {
+        const uint32_t w = sc.list[tid];
+        int rank = 0;
+        for (int j = 0; j < total; ++j) rank += sc.list[j] < w || (sc.list[j] == w && j < tid);
+        sc.sorted[rank] = w;
+      }
+      __syncthreads();
+      // the first of the sorted weights whose sum, itself included, is more than the budget
+      int lo = 0, hi = total;
+      while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        const uint32_t cut = sc.sorted[mid];
+        float mass = 0.f;
+#pragma unroll
+        for (int j = 0; j < OWN; ++j) mass += __float_as_uint(own[j]) <= cut ? own[j] : 0.f;
+        if (row_sum(mass, sc, turn) <= budget) lo = mid + 1;
+        else hi = mid;
+      }
+      const uint32_t tau = lo < total ? min(sc.sorted[lo], one) : one;
+      z = 0.f;
+#pragma unroll
+      for (int j = 0; j < OWN; ++j) {
+        if (__float_as_uint(own[j]) < tau) own[j] = 0.f;
+        z += own[j];
+      }
+      z = row_sum(z, sc, turn);
+    }
+    // multinomial: first token id whose running weight exceeds u * z
+    const float target = u * z;
+    uint32_t weighted = 0;
+#pragma unroll
+    for (int j = 0; j < OWN; ++j)
+      if (chunk[j] >= 0 && own[j] != 0.f) weighted |= 1u << chunk[j];
+    float before[OWN] = {0.f, 0.f, 0.f, 0.f};     // running sums inside the warp
+    for (uint32_t left = __reduce_or_sync(0xffffffffu, weighted); left != 0; left &= left - 1) {
+      const int c = __ffs(left) - 1;
+      float e = 0.f;
+#pragma unroll
+      for (int j = 0; j < OWN; ++j)
+        if (chunk[j] == c) e = own[j];
+      e = warp_running_sum(e);
+#pragma unroll
+      for (int j = 0; j < OWN; ++j)
+        if (chunk[j] == c) before[j] = e;
+      if (lane == 31) sc.chunk_warp[c][warp] = e;
+    }
+    scan_chunks(sc, NV);
+    if (weighted != 0) {
+      float base = 0.f;
+      int c = 0, last = -1, first = 0x7fffffff;
+#pragma unroll
+      for (int j = 0; j < OWN; ++j)
+        if (chunk[j] >= 0 && own[j] > 0.f) {
+          for (; c < chunk[j]; ++c) base += sc.chunk_total[c];
+          last = c * ST + tid;
+          if (first == 0x7fffffff && base + (sc.chunk_warp[c][warp] + before[j]) > target) first = last;
+        }
+      if (first != 0x7fffffff) atomicMin(&sc.choice, first);
+      if (last >= 0) atomicMax(&sc.last, last);
+    }
+    __syncthreads();
+    if (tid == 0) out[b] = sc.choice != 0x7fffffff ? sc.choice : sc.last;
+    return;
+  }
+
+  // every id has a weight
+  float z = 0.f;
+#pragma unroll
+  for (int c = 0; c < NV; ++c) {
+    x[c] = x[c] == -CUDART_INF_F ? 0.f : expf(x[c] - mx);
+    z += x[c];
+  }
+  z = row_sum(z, sc, turn);
+  if (p < 1.f) {
+    const float budget = (1.f - p) * z;
+    uint32_t tau = 0;
+    for (int bit = 30; bit >= 0; --bit) {
+      const uint32_t cand = tau | (1u << bit);
+      if (cand > one) continue;
+      float mass = 0.f;
+#pragma unroll
+      for (int c = 0; c < NV; ++c) mass += __float_as_uint(x[c]) < cand ? x[c] : 0.f;
+      if (row_sum(mass, sc, turn) <= budget) tau = cand;
+    }
+    z = 0.f;
+#pragma unroll
+    for (int c = 0; c < NV; ++c) {
+      if (__float_as_uint(x[c]) < tau) x[c] = 0.f;
+      z += x[c];
+    }
+    z = row_sum(z, sc, turn);
+  }
+  const float target = u * z;
+  uint32_t weighted = 0;      // this thread's chunks with a weight; x becomes the running sum inside the warp
+#pragma unroll
+  for (int c = 0; c < NV; ++c) {
+    if (x[c] > 0.f) weighted |= 1u << c;
+    x[c] = warp_running_sum(x[c]);
+    if (lane == 31) sc.chunk_warp[c][warp] = x[c];
+  }
+  scan_chunks(sc, NV);
+  if (weighted != 0) {
+    float base = 0.f;
+    int first = 0x7fffffff;
+#pragma unroll
+    for (int c = 0; c < NV; ++c) {
+      if ((weighted >> c & 1u) && first == 0x7fffffff && base + (sc.chunk_warp[c][warp] + x[c]) > target) first = c * ST + tid;
+      base += sc.chunk_total[c];
+    }
+    if (first != 0x7fffffff) atomicMin(&sc.choice, first);
+    atomicMax(&sc.last, (31 - __clz(weighted)) * ST + tid);
+  }
+  __syncthreads();
+  if (tid == 0) out[b] = sc.choice != 0x7fffffff ? sc.choice : sc.last;
+}
+
+// The kernel by the length of the rows: registers hold 32 values per thread; longer rows take the passes over `work`.
+static int launch_sample(const char* name, const float* logits, float* work, int n, int v, const float* temperature,
+                         const int* top_k, const float* top_p, const unsigned long long* seeds,
+                         const unsigned long long* counters, int* out, const int* status, cudaStream_t s) {
+  if (v <= 8 * ST)
+    TLLM_LAUNCH(name, sample_row_kernel<8>, n, ST, 0, s, logits, work, v, temperature, top_k, top_p, seeds, counters, out, status);
+  else if (v <= 16 * ST)
+    TLLM_LAUNCH(name, sample_row_kernel<16>, n, ST, 0, s, logits, work, v, temperature, top_k, top_p, seeds, counters, out, status);
+  else if (v <= 32 * ST)
+    TLLM_LAUNCH(name, sample_row_kernel<32>, n, ST, 0, s, logits, work, v, temperature, top_k, top_p, seeds, counters, out, status);
+  else
+    TLLM_LAUNCH(name, sample_kernel, n, ST, 0, s, logits, work, v, temperature, top_k, top_p, seeds, counters, out, status);
+  return TLLM_OK;
 }
 
 }  // namespace tllm
@@ -328,8 +621,7 @@ extern "C" int tllm_sample(const float* logits, float* work, int n, int v, const
                            int* out, const int* status, void* stream) {
   TLLM_REQUIRE(n > 0 && v > 0, "sample: empty input (%d rows of %d)", n, v);
   TLLM_REQUIRE(work != nullptr, "sample: needs n*V floats of scratch");
-  TLLM_LAUNCH("sample", sample_kernel, n, ST, 0, (cudaStream_t)stream, logits, work, v, temperature, top_k, top_p, seeds, counters, out, status);
-  return TLLM_OK;
+  return launch_sample("sample", logits, work, n, v, temperature, top_k, top_p, seeds, counters, out, status, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------- sampling without a caller's scratch
@@ -372,7 +664,6 @@ extern "C" int tllm_sample_noalloc(const float* logits, int n, int v, const floa
     }
     scratch = g_noalloc_ptr[dev];
   }
-  TLLM_LAUNCH("sample_noalloc", sample_kernel, n, ST, 0, (cudaStream_t)stream, logits, scratch, v,
-              temperature, top_k, top_p, seeds, counters, out, (const int*)nullptr);
-  return TLLM_OK;
+  return launch_sample("sample_noalloc", logits, scratch, n, v, temperature, top_k, top_p, seeds, counters, out, nullptr,
+                       (cudaStream_t)stream);
 }
