@@ -761,6 +761,49 @@ def test_sample_top_k_keeps_exactly_k_with_ties(ops):
     assert draws == {5, 9, 50}
 
 
+@pytest.mark.parametrize("nq,nkv,maps,kd,vd", [(8, 1, 1, 64, 64), (6, 2, 1, 48, 64), (5, 5, 2, 64, 32), (8, 2, 1, 128, 128),
+                                               (7, 1, 2, 20, 100)])
+@pytest.mark.parametrize("window,keep,chunk", [(None, 0, None), (300, 0, None), (40, 33, None), (None, 0, 64)])
+def test_attention_of_rows_that_share_their_keys_gives_the_bits_of_one_warp_per_pair(ops, nq, nkv, maps, kd, vd, window, keep, chunk):
+    """32-bit attention with 16 and with 4 rows per CTA against one warp per (token, head): prompts of one and several
+    tiles of rows beside decoded tokens (rows of several requests in one CTA), groups that do not divide the rows, several
+    maps, a sink, a bias by distance, windows with kept keys, chunks, pages given back, and pages that hold NaN where no
+    key is."""
+    g = torch.Generator().manual_seed(nq * 100 + kd)
+    lens, q_lens, page = [700, 5, 97, 64, 1], [1, 5, 40, 1, 1], 8
+    blocks = [-(-n // page) for n in lens]
+    table = torch.full((len(lens), max(blocks)), -1, dtype=torch.int32)
+    ids = torch.randperm(sum(blocks), generator=g).to(torch.int32)
+    kc, vc = torch.full((sum(blocks), nkv * maps, page, kd), math.nan), torch.full((sum(blocks), nkv, page, vd), math.nan)
+    for r, n in enumerate(lens):
+        table[r, :blocks[r]], ids = ids[:blocks[r]], ids[blocks[r]:]
+        for j in range(n):
+            kc[table[r, j // page], :, j % page] = torch.randn(nkv * maps, kd, generator=g)
+            vc[table[r, j // page], :, j % page] = torch.randn(nkv, vd, generator=g)
+        if window and not keep:       # pages behind every window are given back
+            table[r, :max(0, n - q_lens[r] - window) // page] = -1
+    t = sum(q_lens)
+    pos = torch.cat([torch.arange(n - q, n, dtype=torch.int32) for n, q in zip(lens, q_lens)])
+    req = torch.cat([torch.full((q,), r, dtype=torch.int32) for r, q in enumerate(q_lens)])
+    batch = types.SimpleNamespace(token_request=req.to(DEV), positions=pos.to(DEV), max_q_len=max(q_lens))
+    q = (torch.randn(t, nq * maps * kd + 8, generator=g) * 1.5).to(DEV)
+    sink, rel = torch.randn(nq, generator=g).to(DEV), torch.randn(nq, 50, generator=g).to(DEV)
+    for extra in ({}, {"sink": sink, "rel": rel}):
+        outs = []
+        for how in (2, 3, 4, None):
+            out = torch.empty(t, nq * maps * vd, device=DEV)
+            old, ops.generic_attention_split = ops.generic_attention_split, how
+            try:
+                ops.paged_attention_maps(q, nq, nkv, maps, kd, vd, kc.to(DEV), vc.to(DEV), table.to(DEV), batch, out, 0.2,
+                                         window, chunk, keep_first=keep, **extra)
+            finally:
+                ops.generic_attention_split = old
+            outs.append(out)
+        assert bool(torch.isfinite(outs[0]).all())
+        for other in outs[1:]:
+            assert torch.equal(outs[0], other)
+
+
 @pytest.mark.parametrize("vocab", [1, 331, 1024, 1025, 8192, 8193, 16385, 32000, 32768])
 def test_sample_in_registers_draws_what_the_passes_over_memory_draw(ops, vocab):
     """Rows of up to 32,768 logits are kept in registers, longer ones are walked in memory.  A row filled up to 33,000

@@ -16,7 +16,8 @@
 // to lane i mod 8 of eight running softmaxes (m, l, o) in 32-bit, each of which takes its tiles in
 // ascending order; at the end the eight are merged in the order 0..7.  So the order of every sum is a
 // function of p alone: the result does not depend on how the request's tokens were cut into steps, on
-// the rest of the batch or on the page ids.  Two launches of the same arithmetic: with many (token,
+// the rest of the batch or on the page ids.  Launches of the same arithmetic: float32 rows of up to 128 values that share
+// their keys run several to a CTA (paged_attention_rows_kernel, below); else with many (token,
 // head) pairs one warp carries all eight softmaxes of a pair (prompts); with few, eight warps carry
 // one each and merge through shared memory (decoded tokens over a long context, where one warp per
 // pair would leave most of the GPU idle and walk thousands of keys as one chain of memory latencies).
@@ -332,6 +333,346 @@ paged_attention_grouped_kernel(const T* __restrict__ q, int q_row_stride, const 
   }
 }
 
+// ---------------------------------------------------------------- float32: rows that share their keys in one CTA
+// The same arithmetic for R rows at once, a row being a (token, query head of the key row's group) pair and consecutive
+// rows consecutive pairs: a CTA of eight warps, warp w carrying way w of all rows.  What bounded the two launches above was
+// fetching: a lane read its own key row 16 bytes at a time, and every value row was a trip to L2 that the next one waited
+// for.  Here a tile's keys and values come to shared memory by cp.async (the next tile's while this one is worked on),
+// once for all rows; a lane still is a key for the scores and a value column for the output, and the rows go in pairs
+// through fma.rn.f32x2, whose halves round like fmaf.  The sums over a tile's 32 keys keep the tree of warp_sum: partners
+// exchange halves of the rows instead of whole rows, so R rows take R steps of shuffles instead of 5 R.
+// Bound by the reads of shared memory. us per layer at the TinyLlama sizes, this kernel / the launches above: a prompt of
+// 509 tokens 180 / 381, eight decoded tokens at context 700 30 / 68.
+__device__ __forceinline__ uint64_t pack_pair(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack_pair(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// v[r] of all 32 lanes reduced per row r in the tree of the butterflies warp_sum / warp_max (partners 16, 8, 4, 2, 1 apart);
+// lane l gets the result of row l * R / 32.
+template <int R, typename Op>
+__device__ __forceinline__ float reduce_rows(const float (&in)[R], Op op, int lane) {
+  float v[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) v[r] = in[r];
+  int rows = R;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (rows > 1) {
+      rows /= 2;
+      const bool upper = (lane & o) != 0;
+#pragma unroll
+      for (int r = 0; r < R / 2; ++r)
+        if (r < rows) {
+          const float keep = upper ? v[rows + r] : v[r], give = upper ? v[r] : v[rows + r];
+          v[r] = op(keep, __shfl_xor_sync(0xffffffffu, give, o));
+        }
+    } else {
+      v[0] = op(v[0], __shfl_xor_sync(0xffffffffu, v[0], o));
+    }
+  }
+  return v[0];
+}
+
+template <int OD, int R>
+struct RowsSmem {
+  static constexpr bool TWO = OD <= 2;                       // keys and values of a tile in buffers of their own
+  static constexpr int K_LD = OD * 32 + 4, V_LD = OD * 32, P_LD = R + 4;   // pitches that keep 16-byte accesses apart
+  static constexpr int K_FLOATS = 32 * K_LD, V_FLOATS = TWO ? 32 * V_LD : 0, P_FLOATS = 32 * P_LD;
+  static constexpr int WARP_FLOATS = K_FLOATS + V_FLOATS + P_FLOATS;
+  static constexpr int Q_FLOATS = OD * 32 * R;
+  static constexpr int MERGE_LD = OD * 32 + 2;
+  static constexpr int BYTES = (WAYS * WARP_FLOATS + Q_FLOATS) * 4;
+  static_assert(WAYS * R * MERGE_LD <= WAYS * WARP_FLOATS, "the ways' results are parked over the tiles");
+};
+
+template <int OD, int R>   // R = 4 or 16 rows
+__global__ void __launch_bounds__(WAYS * 32)
+paged_attention_rows_kernel(const float* __restrict__ q, int q_row_stride, const float* __restrict__ kcache,
+                            const float* __restrict__ vcache, const int* __restrict__ block_table, int max_blocks,
+                            const int* __restrict__ token_request, const int* __restrict__ positions,
+                            float* __restrict__ out, int n_tokens, Geometry g, float scale, const float* __restrict__ sink) {
+  using S = RowsSmem<OD, R>;
+  extern __shared__ __align__(16) float rows_smem[];
+  __shared__ int pos_s[R], lo_s[R], tok_s[R], head_s[R];   // token -1: no such row
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* q_s = rows_smem;                                   // [key value][row]
+  float* k_s = rows_smem + S::Q_FLOATS + warp * S::WARP_FLOATS;   // [key][K_LD]
+  float* v_s = S::TWO ? k_s + S::K_FLOATS : k_s;            // [key][V_LD]
+  float* p_s = k_s + S::K_FLOATS + S::V_FLOATS;             // [key][P_LD]
+  pdl_trigger();
+  pdl_wait();
+  const int kd = g.kd, vd = g.vd, maps = g.maps, page_size = g.page_size;
+  const int group = g.nq / g.nk, kh = blockIdx.x % g.nk, vh = kh / maps, map = kh % maps;
+  // later tokens see more keys: their tiles start first
+  const long long first = (long long)(gridDim.x / g.nk - 1 - blockIdx.x / g.nk) * R;
+  const long long n_rows = (long long)n_tokens * group;
+  const int t_first = (int)(first / group), t_last = (int)((min(first + R, n_rows) - 1) / group);
+  if (threadIdx.x < R) {
+    const long long row = first + threadIdx.x;
+    const int t = (int)(row / group);
+    const bool ok = row < n_rows;
+    pos_s[threadIdx.x] = ok ? positions[t] : 0;
+    lo_s[threadIdx.x] = ok ? lowest_key(g, positions[t]) : 0;
+    tok_s[threadIdx.x] = ok ? t : -1;
+    head_s[threadIdx.x] = vh * group + (int)(row % group);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < R * kd; i += WAYS * 32) {
+    const int r = i / kd, d = i % kd;
+    const bool ok = tok_s[r] >= 0;
+    q_s[d * R + r] = ok ? q[(size_t)((first + r) / group) * q_row_stride + (size_t)(head_s[r] * maps + map) * kd + d] * scale : 0.f;
+  }
+  __syncthreads();
+
+  uint64_t o[R / 2][OD];
+#pragma unroll
+  for (int r = 0; r < R / 2; ++r)
+#pragma unroll
+    for (int x = 0; x < OD; ++x) o[r][x] = 0ull;
+  const int my_row = lane * R / 32;             // whose maximum and sum this lane keeps
+  float m_run = -CUDART_INF_F, l_run = 0.f;
+
+  // one request at a time (rows of a prompt have one; decoded tokens may have several): the others' rows see no key
+  for (int t = t_first; t <= t_last;) {
+    const int t_begin = t, req = token_request[t];
+    while (t <= t_last && token_request[t] == req) ++t;
+    const int t_end = t;
+    int p_max = -1, p_min = 0x7fffffff, lo_min = 0x7fffffff, lo_max = 0;
+    bool whole = true;                          // every row is of this request
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (tok_s[r] < t_begin || tok_s[r] >= t_end) { whole = false; continue; }
+      p_max = max(p_max, pos_s[r]); p_min = min(p_min, pos_s[r]);
+      lo_min = min(lo_min, lo_s[r]); lo_max = max(lo_max, lo_s[r]);
+    }
+    const int* table = block_table + (size_t)req * max_blocks;
+    const int first_group = (lo_min / (32 * WAYS)) * (32 * WAYS) + warp * 32;
+    auto seen_from = [&](int j0) {              // the first tile of this way from j0 on that some row sees
+      while (j0 <= p_max && !tile_seen(g, j0, lo_min, p_max)) j0 = next_tile(g, j0, 32 * WAYS, first_group);
+      return j0;
+    };
+    // this lane's key of the tile at j0: its page, or -1
+    auto page_of = [&](int j0) {
+      const int j = j0 + lane;
+      return j <= p_max && j / page_size < max_blocks ? table[j / page_size] : -1;
+    };
+    // rows of the tile to shared memory, a row per OD * 8 lanes; keys without a page stay as they are and are not used
+    auto fetch = [&](float* dst, int ld, const float* cache, long long page_stride, long long head_offset, int size, int j0, int page) {
+      constexpr int LANES = OD * 8;
+      const long long off = page < 0 ? -1 : (long long)page * page_stride + head_offset + (long long)((j0 + lane) % page_size) * size;
+      const int c = (lane % LANES) * 4;
+#pragma unroll 4
+      for (int r0 = 0; r0 < 32; r0 += 32 / LANES) {
+        const int r = r0 + lane / LANES;
+        const long long at = __shfl_sync(0xffffffffu, off, r);
+        if (at >= 0 && c < size) copy16_async(dst + r * ld + c, cache + at + c);
+      }
+      copies_commit();
+    };
+    const long long k_head = (long long)kh * g.k_head_stride, v_head = (long long)vh * g.v_head_stride;
+    int j0 = seen_from(g.keep > 0 ? warp * 32 : first_group);
+    int page = j0 <= p_max ? page_of(j0) : -1;
+    if (j0 <= p_max) {
+      fetch(k_s, S::K_LD, kcache, g.k_page_stride, k_head, kd, j0, page);
+      if (S::TWO) fetch(v_s, S::V_LD, vcache, g.v_page_stride, v_head, vd, j0, page);
+    }
+    while (j0 <= p_max) {
+      const int next = seen_from(next_tile(g, j0, 32 * WAYS, first_group));
+      const int next_page = next <= p_max ? page_of(next) : -1;
+      copies_wait<S::TWO ? 1 : 0>();
+      __syncwarp();
+      // ---- scores: this lane's key against all rows
+      uint64_t acc[R / 2];
+#pragma unroll
+      for (int r = 0; r < R / 2; ++r) acc[r] = 0ull;
+      const float* krow = k_s + lane * S::K_LD;
+#pragma unroll 4
+      for (int d = 0; d < kd; d += 4) {
+        const float4 k4 = *reinterpret_cast<const float4*>(krow + d);
+        const float kv[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint64_t kk = pack_pair(kv[e], kv[e]);
+#pragma unroll
+          for (int r = 0; r < R; r += 4) {
+            const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(q_s + (d + e) * R + r);
+            acc[r / 2] = fma_pair(q4.x, kk, acc[r / 2]);
+            acc[r / 2 + 1] = fma_pair(q4.y, kk, acc[r / 2 + 1]);
+          }
+        }
+      }
+      __syncwarp();
+      if (S::TWO) {
+        if (next <= p_max) fetch(k_s, S::K_LD, kcache, g.k_page_stride, k_head, kd, next, next_page);
+        else copies_commit();
+      } else {
+        fetch(v_s, S::V_LD, vcache, g.v_page_stride, v_head, vd, j0, page);
+      }
+      // ---- softmax
+      const int j = j0 + lane;
+      const bool inside = whole && j0 + 31 <= p_min && j0 >= lo_max && __all_sync(0xffffffffu, page >= 0);
+      float s[R], pr[R];
+      uint32_t valid = 0xffffffffu;             // bit r: row r sees this lane's key
+#pragma unroll
+      for (int r = 0; r < R; r += 2) {
+        const float2 two = unpack_pair(acc[r / 2]);
+        s[r] = two.x;
+        s[r + 1] = two.y;
+      }
+      if (!inside) {
+        valid = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (tok_s[r] >= t_begin && tok_s[r] < t_end && page >= 0 && (j >= lo_s[r] || j < g.keep) && j <= pos_s[r]) valid |= 1u << r;
+      }
+      if (g.rel != nullptr) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (valid >> r & 1u) s[r] = biased(g, s[r], head_s[r], pos_s[r] - j);
+      }
+      if (!inside) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (!(valid >> r & 1u)) s[r] = -CUDART_INF_F;
+      }
+      const float m_new = fmaxf(m_run, reduce_rows<R>(s, [](float a, float b) { return fmaxf(a, b); }, lane));
+      const float m_ref = m_new == -CUDART_INF_F ? 0.f : m_new;
+      const float corr = expf(m_run - m_ref);
+      m_run = m_new;
+      bool none = true, every = true;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float ref = __shfl_sync(0xffffffffu, m_ref, r * 32 / R);
+        pr[r] = valid >> r & 1u ? expf(s[r] - ref) : 0.f;
+        none = none && pr[r] == 0.f;
+        every = every && pr[r] != 0.f;
+      }
+      l_run = fmaf(l_run, corr, reduce_rows<R>(pr, [](float a, float b) { return a + b; }, lane));
+#pragma unroll
+      for (int r = 0; r < R; r += 4) *reinterpret_cast<float4*>(p_s + lane * S::P_LD + r) = make_float4(pr[r], pr[r + 1], pr[r + 2], pr[r + 3]);
+      if (!__all_sync(0xffffffffu, corr == 1.f)) {
+#pragma unroll
+        for (int r = 0; r < R; r += 2) {
+          const float c0 = __shfl_sync(0xffffffffu, corr, r * 32 / R), c1 = __shfl_sync(0xffffffffu, corr, (r + 1) * 32 / R);
+#pragma unroll
+          for (int x = 0; x < OD; ++x) {
+            const float2 two = unpack_pair(o[r / 2][x]);
+            o[r / 2][x] = pack_pair(__fmul_rn(two.x, c0), __fmul_rn(two.y, c1));
+          }
+        }
+      }
+      // keys that some row weighs, and keys that every row weighs (the others' products are left out row by row)
+      const uint32_t some = ~__ballot_sync(0xffffffffu, none), all = __ballot_sync(0xffffffffu, every);
+      copies_wait<S::TWO ? 1 : 0>();
+      __syncwarp();
+      // ---- output: this lane's value columns
+      if (all == 0xffffffffu) {
+#pragma unroll 4
+        for (int kk = 0; kk < 32; ++kk) {
+          ulonglong2 p4[R / 4];
+#pragma unroll
+          for (int r = 0; r < R / 4; ++r) p4[r] = *reinterpret_cast<const ulonglong2*>(p_s + kk * S::P_LD + 4 * r);
+#pragma unroll
+          for (int x = 0; x < OD; ++x) {
+            const float v = v_s[kk * S::V_LD + lane + 32 * x];
+            const uint64_t vv = pack_pair(v, v);
+#pragma unroll
+            for (int r = 0; r < R / 4; ++r) {
+              o[2 * r][x] = fma_pair(p4[r].x, vv, o[2 * r][x]);
+              o[2 * r + 1][x] = fma_pair(p4[r].y, vv, o[2 * r + 1][x]);
+            }
+          }
+        }
+      } else {
+        for (uint32_t left = some; left != 0; left &= left - 1) {
+          const int kk = __ffs(left) - 1;
+#pragma unroll
+          for (int x = 0; x < OD; ++x) {
+            const float v = v_s[kk * S::V_LD + lane + 32 * x];
+#pragma unroll
+            for (int r = 0; r < R; r += 2) {
+              const float2 p2 = *reinterpret_cast<const float2*>(p_s + kk * S::P_LD + r);
+              float2 two = unpack_pair(o[r / 2][x]);
+              if (p2.x != 0.f) two.x = fmaf(p2.x, v, two.x);
+              if (p2.y != 0.f) two.y = fmaf(p2.y, v, two.y);
+              o[r / 2][x] = pack_pair(two.x, two.y);
+            }
+          }
+        }
+      }
+      __syncwarp();
+      if (next <= p_max) {
+        if (S::TWO) fetch(v_s, S::V_LD, vcache, g.v_page_stride, v_head, vd, next, next_page);
+        else fetch(k_s, S::K_LD, kcache, g.k_page_stride, k_head, kd, next, next_page);
+      }
+      j0 = next;
+      page = next_page;
+    }
+    copies_wait<0>();
+    __syncwarp();
+  }
+
+  // ---- the ways of every row meet
+  __syncthreads();
+  float* merge_s = rows_smem + S::Q_FLOATS;     // [way][row][MERGE_LD]
+  float* mine = merge_s + warp * R * S::MERGE_LD;
+#pragma unroll
+  for (int r = 0; r < R; r += 2)
+#pragma unroll
+    for (int x = 0; x < OD; ++x) {
+      const float2 two = unpack_pair(o[r / 2][x]);
+      mine[r * S::MERGE_LD + lane + 32 * x] = two.x;
+      mine[(r + 1) * S::MERGE_LD + lane + 32 * x] = two.y;
+    }
+  if (lane % (32 / R) == 0) { mine[my_row * S::MERGE_LD + OD * 32] = m_run; mine[my_row * S::MERGE_LD + OD * 32 + 1] = l_run; }
+  __syncthreads();
+  for (int r = warp; r < R; r += WAYS) {
+    if (tok_s[r] < 0) continue;
+    float sums[OD], l, mx;
+    auto way = [&](int w, int i) { return merge_s[(w * R + r) * S::MERGE_LD + i]; };
+    merge_ways<OD>([&](int w) { return way(w, OD * 32); }, [&](int w) { return way(w, OD * 32 + 1); },
+                   [&](int w, int x) { return way(w, lane + 32 * x); }, sums, l, mx);
+    float* orow = out + (size_t)((first + r) / group) * g.nq * vd + (size_t)(head_s[r] * maps + map) * vd;
+    const float inv = inverse_sum(l, mx, sink, head_s[r]);
+#pragma unroll
+    for (int x = 0; x < OD; ++x)
+      if (lane + 32 * x < vd) orow[lane + 32 * x] = sums[x] * inv;
+  }
+}
+
+template <int OD, int R>
+static int launch_rows(const float* q, int q_row_stride, const float* kcache, const float* vcache, const int* block_table,
+                       int max_blocks, const int* token_request, const int* positions, float* out, int n_tokens,
+                       const Geometry& g, float scale, const float* sink, long long blocks, cudaStream_t s) {
+  auto kern = paged_attention_rows_kernel<OD, R>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RowsSmem<OD, R>::BYTES);
+    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "attention: cannot reserve %d bytes of shared memory: %s", RowsSmem<OD, R>::BYTES, cudaGetErrorString(e));
+    configured = true;
+  }
+  TLLM_LAUNCH("paged_attention_rows", kern, (unsigned)blocks, WAYS * 32, (RowsSmem<OD, R>::BYTES), s, q, q_row_stride, kcache, vcache,
+              block_table, max_blocks, token_request, positions, out, n_tokens, g, scale, sink);
+  return TLLM_OK;
+}
+
 // SPLIT = false: WARPS (token, head) pairs per CTA, one warp each, eight softmaxes in its registers.
 // SPLIT = true: one pair per CTA of eight warps, warp w carries softmax w.
 template <typename T, typename TO, bool SPLIT, int OD>
@@ -448,14 +789,14 @@ using namespace tllm;
 // visible inside the query's chunk of positions only.  out_f32 != 0: the output rows are float32 whatever the cache's type.
 // `sink` (float32, one per query head, or null): exp(sink) joins every softmax's denominator of that head.
 // `keep`: the first positions that a window leaves visible; `rel` (float32 [nq, rel_len] or null): a bias per head and
-// distance.
+// distance.  `max_q_len`: the most tokens of one request in the step (how many rows share their keys; 0 if unknown).
 extern "C" int tllm_paged_attention_maps(const void* q, int q_row_stride, const void* kcache, const void* vcache,
                                          const int* block_table, int max_blocks, const int* token_request,
                                          const int* positions, void* out, int n_tokens, int nq, int nkv, int maps, int kd,
                                          int vd, int page_size, long long k_page_stride, long long k_head_stride,
                                          long long v_page_stride, long long v_head_stride, float scale, int window,
                                          int chunk, int dtype, int out_f32, int split_override, const float* sink,
-                                         int keep, const float* rel, int rel_len, void* stream) {
+                                         int keep, const float* rel, int rel_len, int max_q_len, void* stream) {
   TLLM_REQUIRE(n_tokens > 0 && nq > 0 && nkv > 0 && nq % nkv == 0 && maps > 0,
                "attention: %d tokens, %d heads, %d key/value heads (heads must be a multiple of key/value heads)", n_tokens, nq, nkv);
   TLLM_REQUIRE(kd >= 1 && kd <= MAX_KD && vd >= 1 && vd <= MAX_VD,
@@ -475,7 +816,26 @@ extern "C" int tllm_paged_attention_maps(const void* q, int q_row_stride, const 
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     TLLM_FAIL(TLLM_ERR_CUDA, "attention: cannot read the number of SMs");
-  // split_override: -1 by the number of pairs; 1 eight warps per pair; 0 one warp per (token, key row, four query rows);
+  // Rows that share their keys: a CTA takes 16 of them where that gives every SM one, else 4 (decoded tokens: with 16, half
+  // of the SMs would idle and the chain of one CTA would be longer); fewer than 4 that share keep the launches below.
+  const long long shared_rows = (long long)max_q_len * (nq / nkv), all_rows = (long long)n_tokens * (nq / nkv);
+  const bool vvec = vd % 4 == 0 && ((size_t)vcache % 16) == 0 && v_page_stride % 4 == 0 && v_head_stride % 4 == 0;
+  if (dtype == TLLM_F32 && g.kvec && vvec && kd <= 128 && vd <= 128 &&
+      (split_override < 0 ? shared_rows >= 4 : split_override == 3 || split_override == 4)) {
+    const long long wide = (all_rows + 15) / 16 * g.nk, narrow = (all_rows + 3) / 4 * g.nk;
+    const bool r16 = split_override < 0 ? shared_rows >= 16 && wide >= sms : split_override == 3;
+    TLLM_REQUIRE(narrow <= 2147483647LL, "attention: %lld (token, head) pairs exceed the grid", tasks);
+    cudaStream_t s = (cudaStream_t)stream;
+#define TLLM_ATT_ROWS(OD_, R_)                                                                                         \
+  return launch_rows<OD_, R_>((const float*)q, q_row_stride, (const float*)kcache, (const float*)vcache, block_table,  \
+                              max_blocks, token_request, positions, (float*)out, n_tokens, g, scale, sink,             \
+                              R_ == 16 ? wide : narrow, s)
+    if (kd <= 64 && vd <= 64) { if (r16) TLLM_ATT_ROWS(2, 16); TLLM_ATT_ROWS(2, 4); }
+    if (r16) TLLM_ATT_ROWS(4, 16);
+    TLLM_ATT_ROWS(4, 4);
+#undef TLLM_ATT_ROWS
+  }
+  // split_override: -1 by the number of pairs; 3 and 4: 16 and 4 rows that share their keys (where the sizes allow it); 1 eight warps per pair; 0 one warp per (token, key row, four query rows);
   // 2 one warp per pair (the plainest form, kept for comparison: all give the same bits)
   const bool large = kd > MAX_HD || vd > MAX_HD;
   const bool split = large || (split_override >= 0 ? split_override == 1 : tasks <= 8LL * sms);
@@ -501,7 +861,7 @@ extern "C" int tllm_paged_attention_generic(const void* q, int q_row_stride, con
                                             const int* block_table, int max_blocks, const int* token_request,
                                             const int* positions, void* out, int n_tokens, int nq, int nkv, int hd,
                                             int page_size, long long page_stride, long long head_stride,
-                                            float scale, int window, int dtype, int split_override, void* stream) {
+                                            float scale, int window, int dtype, int split_override, int max_q_len, void* stream) {
   TLLM_REQUIRE(hd >= 16 && hd <= MAX_HD && hd % 16 == 0,
                "attention: head size %d is not built (multiples of 16 up to %d are)", hd, MAX_HD);
   const int elem = dtype == TLLM_F32 ? 4 : 2;
@@ -509,5 +869,5 @@ extern "C" int tllm_paged_attention_generic(const void* q, int q_row_stride, con
                "attention: cache rows must be 16-byte aligned");
   return tllm_paged_attention_maps(q, q_row_stride, kcache, vcache, block_table, max_blocks, token_request, positions, out,
                                    n_tokens, nq, nkv, 1, hd, hd, page_size, page_stride, head_stride, page_stride, head_stride,
-                                   scale, window, 0, dtype, 0, split_override, nullptr, 0, nullptr, 0, stream);
+                                   scale, window, 0, dtype, 0, split_override, nullptr, 0, nullptr, 0, max_q_len, stream);
 }

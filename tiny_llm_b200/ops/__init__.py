@@ -1495,9 +1495,10 @@ def _wide_splits(num_requests: int, num_kv_heads: int, max_kv_len: int) -> int:
     return splits if ctas < lo and hi > 0 and _cluster_merge(num_requests, num_kv_heads, splits) else 0
 
 
-# The attention of the 32-bit path runs eight warps per (token, head) or one warp per (token, key/value head, four query
-# heads), by the number of pairs; both give the same bits.  True / False force one of them, 2 the plainest form (one
-# warp per pair); tests compare the three.
+# The attention of the 32-bit path runs 16 or 4 rows that share their keys per CTA, eight warps per (token, head), or one
+# warp per (token, key/value head, four query heads), by sizes and numbers; all give the same bits.  3 / 4 force the first
+# two (key and value rows of up to 128 values), True / False the others, 2 the plainest form (one warp per pair); tests
+# compare them.
 generic_attention_split = None
 
 
@@ -1584,7 +1585,7 @@ def paged_attention(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, head_d
         _ptr(batch.token_request), _ptr(batch.positions), _ptr(out), t, num_heads, num_kv_heads, head_dim,
         page_size, ctypes.c_longlong(k_cache.stride(0)), ctypes.c_longlong(k_cache.stride(1)),
         ctypes.c_float(scale), int(window or 0), _code(qkv.dtype),
-        -1 if generic_attention_split is None else int(generic_attention_split), _stream())
+        -1 if generic_attention_split is None else int(generic_attention_split), int(getattr(batch, "max_q_len", 0)), _stream())
 
 
 # bfloat16 attention with several score maps per head on the tensor cores (False: the CUDA-core kernel; for measurements)
@@ -1669,7 +1670,7 @@ def paged_attention_maps(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, m
           ctypes.c_longlong(v_cache.stride(0)), ctypes.c_longlong(v_cache.stride(1)), ctypes.c_float(scale),
           int(window or 0), int(chunk or 0), _code(qkv.dtype), 1 if out.dtype == torch.float32 else 0,
           -1 if generic_attention_split is None else int(generic_attention_split), _ptr(sink), keep_first, _ptr(rel), rel_len,
-          _stream())
+          int(getattr(batch, "max_q_len", 0)), _stream())
 
 
 def attention_tc_timing(head_dim: int = 64) -> Optional[dict]:
