@@ -761,6 +761,39 @@ def test_sample_top_k_keeps_exactly_k_with_ties(ops):
     assert draws == {5, 9, 50}
 
 
+@pytest.mark.parametrize("m,nq,nkv,hd,hidden", [
+    (129, 32, 4, 64, 2048),    # tiles of 64 columns
+    (503, 32, 4, 64, 192),     # a depth that does not fill the stages, tiles of 128 columns
+    (257, 9, 3, 64, 320),      # tiles of 64 columns, the last row tile with one row
+    (300, 8, 2, 128, 512),     # tiles of one head of 128
+    (700, 5, 1, 64, 64),       # a single block of K, seven heads
+])
+def test_qkv_projection_in_narrow_tiles(ops, m, nq, nkv, hd, hidden):
+    """Fewer tiles than SMs: they are one or two heads wide.  Queries, keys and
+    values against the plain product, rotated, within bfloat16 rounding (of the product, then of the rotation)."""
+    torch.manual_seed(m)
+    page, pages = 16, -(-m // 16) + 1
+    h, w = torch.randn(m, hidden).bfloat16(), (torch.randn((nq + 2 * nkv) * hd, hidden) * hidden ** -0.5).bfloat16()
+    pos = torch.arange(m, dtype=torch.int32)
+    ang = torch.outer(pos.float(), 10000.0 ** (-torch.arange(hd // 2).float() / (hd // 2)))
+    slots = (torch.randperm(pages - 1)[torch.arange(m) // page] * page + torch.arange(m) % page).to(torch.int32)
+    kc, vc = (torch.zeros(pages, nkv, page, hd, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    out = torch.zeros(m, (nq + 2 * nkv) * hd, dtype=torch.bfloat16, device=DEV)
+    assert ops.linear_rope_kv(h.to(DEV), w.to(DEV), out, pos.to(DEV), ang.cos().to(DEV), ang.sin().to(DEV), nq, nkv, hd,
+                              kc, vc, slots.to(DEV))
+    ref = (h.double() @ w.double().T).view(m, nq + 2 * nkv, hd)
+    c, s = ang.cos().double()[:, None], ang.sin().double()[:, None]
+    lo, hi = ref[..., :hd // 2], ref[..., hd // 2:]
+    turned = torch.cat([lo * c - hi * s, hi * c + lo * s], -1)
+    bound = 3 * 2.0 ** -8 * float(ref.abs().max())      # half a unit for each of x, y and the result, at the largest value
+    assert float((out[:, :nq * hd].cpu().double() - turned[:, :nq].reshape(m, -1)).abs().max()) <= bound
+    at = slots.long()
+    for cache, want in ((kc, turned[:, nq: nq + nkv]), (vc, ref[:, nq + nkv:])):
+        assert float((cache.cpu().double()[at // page, :, at % page] - want).abs().max()) <= bound
+    assert float(kc[pages - 1].abs().sum()) == 0.0       # a page of no token is left alone
+    ops.check_status()
+
+
 @pytest.mark.parametrize("nq,nkv,maps,kd,vd", [(8, 1, 1, 64, 64), (6, 2, 1, 48, 64), (5, 5, 2, 64, 32), (8, 2, 1, 128, 128),
                                                (7, 1, 2, 20, 100)])
 @pytest.mark.parametrize("window,keep,chunk", [(None, 0, None), (300, 0, None), (40, 33, None), (None, 0, 64)])

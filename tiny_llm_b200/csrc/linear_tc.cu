@@ -1025,10 +1025,9 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, void* out, int r
   return TLLM_OK;
 }
 
-template <int EPI>
+template <int EPI, int BN = 256, int STAGES = 4>   // `mb` in boxes of BN rows
 static int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, void* out, int m, int n, int k, int ldo,
                              int* status, cudaStream_t s, const ClusterArgs& ca = ClusterArgs(), const void* w_ptr = nullptr) {
-  constexpr int BN = 256, STAGES = 4;
   using L = PersistentSmem<BN, STAGES>;
   auto kern = linear_tc_persistent_kernel<BN, STAGES, EPI>;
   static bool configured = false;
@@ -1263,8 +1262,19 @@ extern "C" int tllm_linear_tc_cluster(const void* a, const void* w, void* out, i
   if (m > 128) {
     // many tokens: 128 x 256 tiles of C as in tllm_linear_tc, with the rotation and the cache write in the epilogue
     TLLM_REQUIRE(hd == 64 || hd == 128, "linear_tc_cluster: the Q/K/V epilogue for more than 128 tokens takes head size 64 or 128 (got %d)", hd);
-    if (!make_map(&ma, a, m, k, lda, BM) || !make_map(&mb, w, n, k, k, 256))
+    // With fewer tiles than SMs the time is that of one tile: a chain of k-blocks, each 1.1 us away from memory with four
+    // of 48 KB in flight (0.35 us per k-block).  Narrower tiles put more SMs to work and leave room for more stages: the
+    // narrowest (whole heads) that give at most one tile to an SM.  20 tiles of 256 as 80 of 64 (2,560 x 2,048, 131 tokens)
+    // 20 -> 15 us, 40 as 80 of 128 (503 tokens) 20 -> 17; the same widths as strips with four stages gained 4 and 1 us.
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      TLLM_FAIL(TLLM_ERR_CUDA, "linear_tc_cluster: cannot read the number of SMs");
+    const long long tiles_m = (m + BM - 1) / BM;
+    const int width = hd == 64 && tiles_m * ((n + 63) / 64) <= sms ? 64 : (tiles_m * ((n + 127) / 128) <= sms ? 128 : 256);
+    if (!make_map(&ma, a, m, k, lda, BM) || !make_map(&mb, w, n, k, k, width))
       TLLM_FAIL(TLLM_ERR_CUDA, "linear_tc_cluster: cuTensorMapEncodeTiled failed");
+    if (width == 64) return launch_persistent<EPI_ROPE_KV, 64, 7>(ma, mb, out, m, n, k, ldo, status, s, ca, w);
+    if (width == 128) return launch_persistent<EPI_ROPE_KV, 128, 6>(ma, mb, out, m, n, k, ldo, status, s, ca, w);
     return launch_persistent<EPI_ROPE_KV>(ma, mb, out, m, n, k, ldo, status, s, ca, w);
   }
   const int bn = m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : 128));
