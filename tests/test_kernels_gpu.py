@@ -286,6 +286,25 @@ def test_paged_attention(ops, dtype, nq, nkv, hd, page, window):
         assert float(p[3]) > 0.9
 
 
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(1, 4), (129, 36), (2049, 1028), (8192, 260), (8205, 2048)])
+def test_float32_products_of_few_rows_stream_any_shape(ops, m, n, k, monkeypatch):
+    """Every shape of the streaming kernel (rows of A that fill no group, weight rows that fill no CTA, on both sides of
+    the line between the shapes, depths of one piece, of a part of a box, of more boxes than the ring holds), rows of A
+    inside wider ones: the bits of the tile kernel."""
+    torch.manual_seed(m * 7 + n)
+    a, w = torch.randn(m, k + 12, device=DEV)[:, 4:k + 4], torch.randn(n, k, device=DEV)
+    outs = []
+    for streamed in (True, False):
+        monkeypatch.setattr(ops, "linear_skinny", streamed)
+        out, acc = torch.full((m, n + 1), 3.0, device=DEV), torch.full((m, n), -0.5, device=DEV)
+        ops.linear(a, w, out[:, :n])
+        ops.linear(a, w, acc, accumulate=True)
+        outs.append((out, acc))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    ops.check_status()
+
+
 @pytest.mark.parametrize("m,n,k", [(17, 64, 4), (17, 2561, 20), (33, 4801, 36), (100, 2560, 64), (65, 9473, 16), (509, 2560, 40),
                                    (64, 12161, 68), (513, 130, 1028)])
 def test_float32_tiles_of_every_size_give_the_bits_of_the_tile_kernel(ops, m, n, k, monkeypatch):

@@ -5,14 +5,13 @@
 // so a row's result does not depend on its batch, to the bit.
 //   linear_generic_kernel: 64 x 64 tiles, 4 x 4 outputs per thread (any sizes and both dtypes);
 //   linear_tiled_kernel: float32, more than 16 rows, rows on 16 bytes: tiles from 16 x 64 to 64 x 192 by the sizes;
-//   linear_skinny_kernel: float32, at most 16 rows (decoded tokens): a CTA takes 8 or 16 weight rows and
-//     streams them through shared memory in chunks of 128 k (cp.async, three stages), one thread per
-//     output element.  With so few rows the 64-row tile left 32 CTAs to stream a matrix that 148 SMs could
-//     pull, each with one load in flight per thread.
+//   linear_skinny_kernel: float32, at most 16 rows (decoded tokens), rows on 16 bytes: the weights stream through a ring
+//     of TMA boxes.
+// A bounded wait that runs out leaves a code in the device's status word.
 // Reference counterpart: tiny_llm/ops/cuda/gemm.cu:67-106 (64x256 tile, 8x8 outputs per thread).
 #include <cstdint>
 
-#include "common.cuh"
+#include "tc_common.cuh"
 
 TLLM_DEFINE_LAST_ERROR
 
@@ -297,97 +296,193 @@ static int launch_tiled(const float* a, const float* w, float* out, int m, int n
 }
 
 // ---------------------------------------------------------------- at most 16 rows, float32
-constexpr int SK_KC = 128, SK_LD = SK_KC + 4, SK_STAGES = 3, SK_THREADS = 128;
-
-__device__ __forceinline__ void sk_cp16(float* dst, const float* src, bool ok) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  const int bytes = ok ? 16 : 0;   // 0: the 16 bytes are filled with zeros, which leave a chain of fmaf as it is
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+// A CTA streams ROWS = W x RW weight rows and the R rows of A through a ring of TMA boxes of 32 k (128-byte swizzle: rows
+// lie 128 bytes apart and 16-byte reads of eight rows do not collide), KB boxes per stage; a producer warp issues them,
+// the weights' first stages before the wait for earlier kernels.  A lane owns one weight row and TR rows of A: TR chains of
+// fmaf, whose operands it reads KS steps of four k ahead (read where they are used, every step stood behind a trip to
+// shared memory).  What bounds it: the weights from memory where there are many rows of them, else the reads of shared
+// memory (1 + TR per four k); the chains themselves (4 cycles per k) would take 4.3 us at K = 2,048.
+// us, this kernel / one chain per thread with cp.async by the computing threads (m = 8): 2,560 x 2,048 14.9 / 26.8,
+// 2,048 x 2,048 13.8 / 20.2, 11,264 x 2,048 27.4 / 43.5, 2,048 x 5,632 34.2 / 55.0, 32,000 x 2,048 74.6 / 115.7; m = 1:
+// 9.0 / 18.3, 8.5 / 17.4, 23.8 / 26.9, 19.9 / 43.2, 46.9 / 50.0.
+__device__ __forceinline__ float4 read_shared4(uint32_t at) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+  return v;
 }
-template <int R, int MODE>   // R rows of A per CTA (1, 2, 4, 8 or 16); BNS weight rows: R x BNS = at most 128 threads compute
-__global__ void __launch_bounds__(SK_THREADS)
-linear_skinny_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ out,
-                     int m, int n, int k, int lda, int ldo) {
-  constexpr int BNS = R == 16 ? 8 : 16;
-  extern __shared__ __align__(16) uint8_t sk_smem[];
-  float (*w_s)[BNS][SK_LD] = reinterpret_cast<float (*)[BNS][SK_LD]>(sk_smem);
-  float (*a_s)[R][SK_LD] = reinterpret_cast<float (*)[R][SK_LD]>(sk_smem + sizeof(float) * SK_STAGES * BNS * SK_LD);
-  pdl_trigger();
-  const int tid = threadIdx.x;
-  const int n0 = blockIdx.x * BNS, m0 = blockIdx.y * R;
-  const int chunks = (k + SK_KC - 1) / SK_KC;
-  auto load_w = [&](int chunk, int stage) {
-    const int k0 = chunk * SK_KC;
-    for (int idx = tid; idx < BNS * (SK_KC / 4); idx += SK_THREADS) {
-      const int row = idx / (SK_KC / 4), kk = (idx % (SK_KC / 4)) * 4;
-      const bool ok = n0 + row < n && k0 + kk < k;   // k is a multiple of 4
-      sk_cp16(&w_s[stage][row][kk], ok ? w + (size_t)(n0 + row) * k + k0 + kk : w, ok);
-    }
-  };
-  auto load_a = [&](int chunk, int stage) {
-    const int k0 = chunk * SK_KC;
-    for (int idx = tid; idx < R * (SK_KC / 4); idx += SK_THREADS) {
-      const int row = idx / (SK_KC / 4), kk = (idx % (SK_KC / 4)) * 4;
-      const bool ok = m0 + row < m && k0 + kk < k;
-      sk_cp16(&a_s[stage][row][kk], ok ? a + (size_t)(m0 + row) * lda + k0 + kk : a, ok);
-    }
-  };
-  // the weights depend on no earlier kernel: their first chunks are on the way before the wait
-  for (int st = 0; st < SK_STAGES - 1; ++st)
-    if (st < chunks) load_w(st, st);
-  pdl_wait();
-  for (int st = 0; st < SK_STAGES - 1; ++st) {
-    if (st < chunks) load_a(st, st);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+constexpr int ERR_SK_PRODUCER = 1, ERR_SK_CONSUMER = 3;
+
+template <int R, int RW, int TR, int W, int KB, int ST>
+struct Skinny {
+  static constexpr int ROWS = W * RW, GROUPS = R / TR, KC = KB * 32;
+  static_assert(GROUPS * TR == R && GROUPS * RW <= 32 && ROWS % 8 == 0, "lanes of a warp; whole swizzle atoms");
+  static constexpr int W_BOX = ROWS * 128, A_BOX = R * 128, A_STEP = A_BOX < 1024 ? 1024 : A_BOX;
+  static constexpr int STAGE = KB * (W_BOX + A_STEP);
+  static constexpr int SMEM = ST * STAGE + 2 * ST * 8 + 16 + 1024;   // + alignment slack
+};
+
+template <int R, int RW, int TR, int W, int KB, int ST, int MODE>
+__global__ void __launch_bounds__(W * 32 + 32)
+linear_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
+                     float* __restrict__ out, int m, int n, int k, int ldo, int* __restrict__ status) {
+  using C = Skinny<R, RW, TR, W, KB, ST>;
+  extern __shared__ uint8_t sk_smem[];
+  uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(sk_smem) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = reinterpret_cast<uint64_t*>(sm + ST * C::STAGE);
+  uint64_t* empty = full + ST;
+  volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(empty + ST);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n0 = blockIdx.x * C::ROWS, m0 = blockIdx.y * R;
+  const int chunks = (k + C::KC - 1) / C::KC;
+  if (tid == 0) {
+    tma_prefetch_map(&map_w);
+    tma_prefetch_map(&map_a);
+    for (int s = 0; s < ST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], W); }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  const bool computes = tid < R * BNS;
-  const int r = tid / BNS, c = tid % BNS;
-  float acc = 0.f;
-  for (int i = 0; i < chunks; ++i) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(SK_STAGES - 2) : "memory");
-    __syncthreads();   // chunk i has landed for every thread, and everyone has left chunk i - 1, whose stage is refilled now
-    const int nxt = i + SK_STAGES - 1;
-    if (nxt < chunks) { load_w(nxt, nxt % SK_STAGES); load_a(nxt, nxt % SK_STAGES); }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    if (computes) {
-      const float* ar = a_s[i % SK_STAGES][r];
-      const float* wr = w_s[i % SK_STAGES][c];
-#pragma unroll 8
-      for (int kk = 0; kk < SK_KC; kk += 4) {
-        const float4 av = *reinterpret_cast<const float4*>(ar + kk);
-        const float4 wv = *reinterpret_cast<const float4*>(wr + kk);
-        acc = fmaf(av.x, wv.x, acc);
-        acc = fmaf(av.y, wv.y, acc);
-        acc = fmaf(av.z, wv.z, acc);
-        acc = fmaf(av.w, wv.w, acc);
+  __syncthreads();
+  pdl_trigger();
+
+  if (warp == W) {
+    // ---------------- producer
+    if (lane == 0) {
+      auto load_w = [&](int c) {
+        const int s = c % ST;
+        mbar_expect_tx(&full[s], KB * (C::W_BOX + C::A_BOX));
+#pragma unroll
+        for (int b = 0; b < KB; ++b) tma_load_2d(sm + s * C::STAGE + b * C::W_BOX, &map_w, c * C::KC + b * 32, n0, &full[s]);
+      };
+      auto load_a = [&](int c) {
+        const int s = c % ST;
+#pragma unroll
+        for (int b = 0; b < KB; ++b)
+          tma_load_2d(sm + s * C::STAGE + KB * C::W_BOX + b * C::A_STEP, &map_a, c * C::KC + b * 32, m0, &full[s]);
+      };
+      const int pre = min(chunks, ST);
+      for (int c = 0; c < pre; ++c) load_w(c);
+      pdl_wait();
+      for (int c = 0; c < pre; ++c) load_a(c);
+      for (int c = ST; c < chunks; ++c) {
+        if (!mbar_wait(&empty[c % ST], ((c / ST) & 1) ^ 1, abort_flag)) { *abort_flag = 1; atomicExch(status, ERR_SK_PRODUCER); break; }
+        load_w(c);
+        load_a(c);
       }
     }
+    return;
   }
-  const int gm = m0 + r, gn = n0 + c;
-  if (computes && gm < m && gn < n) {
-    const size_t o = (size_t)gm * ldo + gn;
-    if (MODE == OUT_ACC) out[o] += acc;
-    else out[o] = acc;
+
+  // ---------------- computing warps
+  pdl_wait();
+  const bool computes = lane < RW * C::GROUPS;
+  const int row = warp * RW + lane % RW, group = computes ? lane / RW : 0;   // weight row; rows of A group * TR + i
+  uint32_t w_at[8], a_at[TR][8];                                             // 16-byte pieces of a box, unswizzled
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    w_at[j] = (uint32_t)(row * 128 + ((j ^ (row & 7)) << 4));
+#pragma unroll
+    for (int i = 0; i < TR; ++i) a_at[i][j] = (uint32_t)((group * TR + i) * 128 + ((j ^ ((group * TR + i) & 7)) << 4));
+  }
+  float acc[TR];
+#pragma unroll
+  for (int i = 0; i < TR; ++i) acc[i] = 0.f;
+  constexpr int KS = TR <= 2 ? 4 : (TR <= 4 ? 2 : 1), BLOCKS = C::KC / 4 / KS;
+  for (int c = 0; c < chunks; ++c) {
+    const bool ok = mbar_wait(&full[c % ST], (c / ST) & 1, abort_flag);
+    if (!__all_sync(0xffffffffu, ok)) {
+      if (lane == 0) { *abort_flag = 1; atomicExch(status, ERR_SK_CONSUMER); }
+      return;
+    }
+    const uint32_t wb = smem_u32(sm) + (c % ST) * C::STAGE, ab = wb + KB * C::W_BOX;
+    float4 wv[2][KS], av[2][KS][TR];
+    auto read = [&](int block) {
+#pragma unroll
+      for (int j = 0; j < KS; ++j) {
+        const int piece = block * KS + j;
+        wv[block & 1][j] = read_shared4(wb + piece / 8 * C::W_BOX + w_at[piece % 8]);
+#pragma unroll
+        for (int i = 0; i < TR; ++i) av[block & 1][j][i] = read_shared4(ab + piece / 8 * C::A_STEP + a_at[i][piece % 8]);
+      }
+    };
+    read(0);
+#pragma unroll
+    for (int block = 0; block < BLOCKS; ++block) {
+      if (block + 1 < BLOCKS) read(block + 1);
+#pragma unroll
+      for (int j = 0; j < KS; ++j) {
+        const float4 w4 = wv[block & 1][j];
+        const float4* a4 = av[block & 1][j];
+#pragma unroll
+        for (int i = 0; i < TR; ++i) acc[i] = fmaf(a4[i].x, w4.x, acc[i]);
+#pragma unroll
+        for (int i = 0; i < TR; ++i) acc[i] = fmaf(a4[i].y, w4.y, acc[i]);
+#pragma unroll
+        for (int i = 0; i < TR; ++i) acc[i] = fmaf(a4[i].z, w4.z, acc[i]);
+#pragma unroll
+        for (int i = 0; i < TR; ++i) acc[i] = fmaf(a4[i].w, w4.w, acc[i]);
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[c % ST]);
+  }
+  if (!computes || n0 + row >= n) return;
+#pragma unroll
+  for (int i = 0; i < TR; ++i) {
+    const int gm = m0 + group * TR + i;
+    if (gm >= m) continue;
+    const size_t o = (size_t)gm * ldo + n0 + row;
+    if (MODE == OUT_ACC) out[o] += acc[i];
+    else out[o] = acc[i];
   }
 }
 
-template <int R>
-int launch_skinny(const float* a, const float* w, float* out, int m, int n, int k, int lda, int ldo, int mode, cudaStream_t s) {
-  constexpr int BNS = R == 16 ? 8 : 16;
-  constexpr int SMEM = (int)sizeof(float) * SK_STAGES * (BNS + R) * SK_LD;   // at most 38 KB
+// A float32 matrix [rows, k] with row stride ld, in boxes of `box` rows x 32 values.
+static bool make_skinny_map(CUtensorMap* map, const float* ptr, int rows, int k, long long ld, int box) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  cuuint32_t boxes[2] = {32u, (cuuint32_t)box};
+  cuuint32_t elem[2] = {1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(ptr), dims, strides, boxes, elem,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int R, int RW, int TR, int W, int KB, int ST>
+int launch_skinny(const float* a, const float* w, float* out, int m, int n, int k, int lda, int ldo, int mode, int* status, cudaStream_t s) {
+  using C = Skinny<R, RW, TR, W, KB, ST>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(linear_skinny_kernel<R, OUT_ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_skinny_kernel<R, OUT_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "linear_skinny: cannot reserve %d bytes of shared memory: %s", SMEM, cudaGetErrorString(e));
+    cudaError_t e = cudaFuncSetAttribute(linear_skinny_kernel<R, RW, TR, W, KB, ST, OUT_ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_skinny_kernel<R, RW, TR, W, KB, ST, OUT_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "linear_skinny: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
     configured = true;
   }
-  dim3 grid((n + BNS - 1) / BNS, (m + R - 1) / R);
+  CUtensorMap mw, ma;
+  if (!make_skinny_map(&mw, w, n, k, k, C::ROWS) || !make_skinny_map(&ma, a, m, k, lda, R))
+    TLLM_FAIL(TLLM_ERR_CUDA, "linear_skinny: cuTensorMapEncodeTiled failed");
+  dim3 grid((n + C::ROWS - 1) / C::ROWS, (m + R - 1) / R);
   if (mode == OUT_ACC)
-    TLLM_LAUNCH("linear_skinny", (linear_skinny_kernel<R, OUT_ACC>), grid, SK_THREADS, SMEM, s, a, w, out, m, n, k, lda, ldo);
+    TLLM_LAUNCH("linear_skinny", (linear_skinny_kernel<R, RW, TR, W, KB, ST, OUT_ACC>), grid, W * 32 + 32, C::SMEM, s, mw, ma, out, m, n, k, ldo, status);
   else
-    TLLM_LAUNCH("linear_skinny", (linear_skinny_kernel<R, OUT_F32>), grid, SK_THREADS, SMEM, s, a, w, out, m, n, k, lda, ldo);
+    TLLM_LAUNCH("linear_skinny", (linear_skinny_kernel<R, RW, TR, W, KB, ST, OUT_F32>), grid, W * 32 + 32, C::SMEM, s, mw, ma, out, m, n, k, ldo, status);
   return TLLM_OK;
+}
+
+// Which shape: few weight rows want small CTAs (more SMs at work), many want the weight rows' reads shared by more rows of A
+// (8 x 11,264 x 2,048: 16 weight rows per warp 27.4 us, 8 41.9; 8 x 2,048 x 2,048: 20 and 13.8; the line between at
+// 8,192 weight rows is where both leave no SM idle).
+static int launch_skinny_rows(const float* a, const float* w, float* out, int m, int n, int k, int lda, int ldo, int mode, int* status, cudaStream_t s) {
+  const bool many = n >= 8192;
+  if (m <= 1) return many ? launch_skinny<1, 32, 1, 1, 2, 8>(a, w, out, m, n, k, lda, ldo, mode, status, s)
+                          : launch_skinny<1, 16, 1, 1, 4, 8>(a, w, out, m, n, k, lda, ldo, mode, status, s);
+  if (m <= 2) return launch_skinny<2, 16, 1, 2, 4, 5>(a, w, out, m, n, k, lda, ldo, mode, status, s);
+  if (m <= 4) return launch_skinny<4, 8, 1, 2, 4, 6>(a, w, out, m, n, k, lda, ldo, mode, status, s);
+  if (m <= 8) return many ? launch_skinny<8, 16, 4, 2, 2, 6>(a, w, out, m, n, k, lda, ldo, mode, status, s)
+                          : launch_skinny<8, 8, 2, 1, 4, 6>(a, w, out, m, n, k, lda, ldo, mode, status, s);
+  return many ? launch_skinny<16, 16, 8, 2, 2, 6>(a, w, out, m, n, k, lda, ldo, mode, status, s)
+              : launch_skinny<16, 8, 4, 2, 4, 5>(a, w, out, m, n, k, lda, ldo, mode, status, s);
 }
 
 template <typename T>
@@ -408,21 +503,17 @@ int launch(const void* a, const void* w, void* out, int m, int n, int k, int lda
 
 // skinny: 0 keeps the 64 x 64 tile kernel for every size (tests compare it with the two others, which must agree with it to the bit)
 extern "C" int tllm_linear_generic(const void* a, const void* w, void* out, int m, int n, int k, int lda, int ldo,
-                                   int dtype, int mode, int skinny, void* stream) {
+                                   int dtype, int mode, int skinny, int* status, void* stream) {
   TLLM_REQUIRE(m > 0 && n > 0 && k > 0, "linear: empty product %d x %d x %d", m, n, k);
   TLLM_REQUIRE(lda >= k && ldo >= n, "linear: row strides %d, %d are shorter than the rows %d, %d", lda, ldo, k, n);
   TLLM_REQUIRE((m + tllm::BM - 1) / tllm::BM <= 65535, "linear: %d rows exceed the grid", m);
-  if (dtype == TLLM_F32 && m <= 16 && skinny != 0 && k % 4 == 0 && lda % 4 == 0 && ((uintptr_t)a % 16) == 0 && ((uintptr_t)w % 16) == 0 &&
+  if (dtype == TLLM_F32 && m <= 16 && skinny != 0 && status != nullptr && k % 4 == 0 && lda % 4 == 0 && ((uintptr_t)a % 16) == 0 && ((uintptr_t)w % 16) == 0 &&
       (mode == tllm::OUT_SAME || mode == tllm::OUT_F32 || mode == tllm::OUT_ACC)) {
     const float* af = (const float*)a;
     const float* wf = (const float*)w;
     float* of = (float*)out;
     cudaStream_t s = (cudaStream_t)stream;
-    if (m <= 1) return tllm::launch_skinny<1>(af, wf, of, m, n, k, lda, ldo, mode, s);
-    if (m <= 2) return tllm::launch_skinny<2>(af, wf, of, m, n, k, lda, ldo, mode, s);
-    if (m <= 4) return tllm::launch_skinny<4>(af, wf, of, m, n, k, lda, ldo, mode, s);
-    if (m <= 8) return tllm::launch_skinny<8>(af, wf, of, m, n, k, lda, ldo, mode, s);
-    return tllm::launch_skinny<16>(af, wf, of, m, n, k, lda, ldo, mode, s);
+    return tllm::launch_skinny_rows(af, wf, of, m, n, k, lda, ldo, mode, status, s);
   }
   if (dtype == TLLM_F32 && skinny != 0 && m > 16 && k % 4 == 0 && lda % 4 == 0 && ((uintptr_t)a % 16) == 0 && ((uintptr_t)w % 16) == 0 &&
       n <= 64 * 65535 && (mode == tllm::OUT_SAME || mode == tllm::OUT_F32 || mode == tllm::OUT_ACC))

@@ -1388,7 +1388,7 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool
         return
     lib = build.load_library("linear_generic")
     _call(lib, lib.tllm_linear_generic, _ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0), out.stride(0),
-                                        _code(a.dtype), mode, int(linear_skinny), _stream())
+                                        _code(a.dtype), mode, int(linear_skinny), _ptr(status_word(a.device)), _stream())
 
 
 def linear_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, block: int, workspace,
