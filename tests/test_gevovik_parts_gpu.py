@@ -317,6 +317,37 @@ def test_delta_rule_with_a_decay_per_key_channel(sizes):
         assert torch.equal(a, b)     # the same operations on every state element however the sequence is cut
 
 
+@pytest.mark.parametrize("mode", ["delta", "state_space", "channel_decay"])
+@pytest.mark.parametrize("sizes", [(2, 1, 4, 5), (4, 2, 36, 16), (3, 3, 64, 33), (4, 1, 128, 48), (2, 2, 252, 20)])
+def test_streamed_recurrence_gives_the_bits_of_the_general_kernel(mode, sizes):
+    """Key rows on 16 bytes take the streamed kernel, rows that start elsewhere the general one: the same operations on
+    every state element.  Requests of no, one, seven, eight, nine and more tokens than the ring holds."""
+    from tiny_llm_b200 import ops
+    heads, kvh, kd, vd = sizes
+    lens = [0, 1, 7, 8, 9, 77]
+    g, n = torch.Generator().manual_seed(kd + len(mode)), sum(lens)
+    q, k, v = (x.reshape(n, -1).contiguous() for x in recurrence_inputs(g, n, heads, kvh, kd, vd))
+    gb = torch.rand(n, heads, 2, generator=g) * 0.9 + 0.05
+    gk = torch.rand(n, heads * kd, generator=g) if mode == "channel_decay" else None
+    if gk is not None:
+        gb[..., 0] = 1.0
+    states = torch.randn(len(lens), heads, vd, kd, generator=g)
+    b = batch_of(lens, [0] * len(lens))
+
+    def off(x):       # the same values four bytes past a 16-byte boundary
+        y = torch.empty(x.numel() + 1, device=DEV)
+        y[1:] = x.to(DEV).reshape(-1)
+        return y[1:].view(x.shape)
+    got = []
+    for place in (lambda x: x.to(DEV), off):
+        state, out = states.clone().to(DEV), torch.zeros(n, heads * vd, device=DEV)
+        ops.delta_rule_scan(place(q), place(k), v.to(DEV), gb.to(DEV), state, b, heads, kvh, kd, vd, out, mode=mode,
+                            gk=None if gk is None else place(gk))
+        got.append((out, state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    ops.check_status()
+
+
 @pytest.mark.parametrize("sizes", [(4, 2, 16, 16), (6, 3, 10, 6), (5, 5, 12, 8), (2, 1, 7, 20), (8, 2, 64, 32), (16, 16, 32, 8)])
 def test_state_space_recurrence_and_the_gated_norm_in_parts(sizes):
     from tiny_llm_b200 import ops

@@ -27,7 +27,9 @@
 //   memory eight at a time by cp.async, the next eight in flight meanwhile.  The state is kept transposed
 //   ([slot, head, value column, key row]) so that a group's rows are consecutive in memory.  What is done to a state
 //   element is the same sequence of operations however the request was cut into steps: the same bits.
-#include "common.cuh"
+// delta_rule_stream: the same for key rows of whole 16-byte pieces.  A bounded wait that runs out leaves a code in the
+//   device's status word.
+#include "tc_common.cuh"
 
 TLLM_DEFINE_LAST_ERROR
 
@@ -327,6 +329,236 @@ __global__ void __launch_bounds__(128) delta_rule_scan_kernel(ScanArgs a) {
 }
 
 
+// The same recurrence, to the bit, where a key row is whole 16-byte pieces.  What bounded the kernel above was not its chain
+// per token (two rounds of products and three of shuffles, about 150 cycles) but what stood between the chains: the
+// copies' address arithmetic in every thread, two block barriers per eight tokens, three sums shuffled where the chain
+// needs one.  Here a producer warp fills a ring of stages of eight tokens (a 16-byte piece of a row per lane), state rows
+// go in pairs through fma.rn.f32x2, the tokens' values, decays and step sizes wait in registers, a token per lane, for a
+// shuffle, and what only the read-out needs is summed for eight tokens at once.  (Two columns per lane, which halve the
+// reads of shared memory, were slower, 378 us against 335: the chain then carries twice the products.)
+// us for 1,777 tokens of 128 x 128, this kernel / the one above: mode 0, 16 heads 278 / 391; mode 1, 32 heads 328 / 450;
+// mode 2, 16 heads 332 / 447; keys of 200, mode 2, 200 tokens 36 / 196; 61 tokens 18 / 24.
+__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 halves_of(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {   // each half rounds like fmaf
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+constexpr int DR_STAGES = 4, ERR_DR_PRODUCER = 1, ERR_DR_CONSUMER = 3;
+
+template <int R, int MODE>
+struct Stream {
+  static constexpr int WARPS = DR_COLS * DR_LANES / 32;
+  static constexpr int ARRAYS = MODE == 2 ? 3 : 2, CH = R + 4, ROW = CH * DR_LANES;   // a lane's part of a staged row, padded (see above); the row
+  static constexpr int STAGE = ARRAYS * DR_TOK * ROW;
+  static constexpr int SMEM = DR_STAGES * STAGE * 4 + 2 * DR_STAGES * 8 + 16;
+};
+
+// x[t] of the eight lanes of a group summed per t in the tree of shuffles 4, 2, 1 apart; lane `sub` gets the sum of x[sub].
+__device__ __forceinline__ float sum_per_token(float (&x)[DR_TOK], int sub) {
+  static_assert(DR_TOK == 8 && DR_LANES == 8, "a token per lane");
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    const bool upper = (sub & o) != 0;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float keep = upper ? x[o + i] : x[i], give = upper ? x[i] : x[o + i];
+      x[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  return x[0];
+}
+
+template <int R, int MODE>   // R * DR_LANES >= key size
+__global__ void __launch_bounds__(Stream<R, MODE>::WARPS * 32 + 32) delta_rule_stream_kernel(ScanArgs a, int* __restrict__ status) {
+  using C = Stream<R, MODE>;
+  extern __shared__ __align__(16) float dr_smem[];     // [stage][keys, queries, decays][token][ROW]
+  uint64_t* full = reinterpret_cast<uint64_t*>(dr_smem + DR_STAGES * C::STAGE);
+  uint64_t* empty = full + DR_STAGES;
+  volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(empty + DR_STAGES);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = blockIdx.y, req = blockIdx.z, kh = h / (a.heads / a.kv_heads);
+  if (tid == 0) {
+    for (int s = 0; s < DR_STAGES; ++s) { mbar_init(&full[s], 32); mbar_init(&empty[s], C::WARPS); }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (a.kd < R * DR_LANES)      // rows past the key size stay zero
+    for (int i = tid; i < DR_STAGES * C::STAGE; i += C::WARPS * 32 + 32) dr_smem[i] = 0.f;
+  __syncthreads();
+  pdl_trigger();
+  pdl_wait();
+  const int t0 = a.cu_q[req], t1 = a.cu_q[req + 1], stages = (t1 - t0 + DR_TOK - 1) / DR_TOK;
+
+  if (warp == C::WARPS) {
+    // ---------------- producer: a lane copies the same pieces of every row
+    const size_t qk_ld = (size_t)a.kv_heads * a.kd, g_ld = (size_t)a.heads * a.kd;
+    for (int i = 0; i < stages; ++i) {
+      const int s = i % DR_STAGES, tb = t0 + i * DR_TOK, nt = min(DR_TOK, t1 - tb);
+      const bool ok = i < DR_STAGES || mbar_wait(&empty[s], ((i / DR_STAGES) & 1) ^ 1, abort_flag);
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) { *abort_flag = 1; atomicExch(status, ERR_DR_PRODUCER); }
+        break;
+      }
+      float* stage = dr_smem + s * C::STAGE;
+#pragma unroll
+      for (int d = lane * 4; d < R * DR_LANES; d += 128) {
+        if (d >= a.kd) break;
+        const int at = d / R * C::CH + d % R;
+        const size_t qk = (size_t)tb * qk_ld + (size_t)kh * a.kd + d, gd = (size_t)tb * g_ld + (size_t)h * a.kd + d;
+        for (int tt = 0; tt < nt; ++tt) {
+          cp_async16(stage + tt * C::ROW + at, a.k + qk + tt * qk_ld);
+          cp_async16(stage + (DR_TOK + tt) * C::ROW + at, a.q + qk + tt * qk_ld);
+          if (MODE == 2) cp_async16(stage + (2 * DR_TOK + tt) * C::ROW + at, a.gk + gd + tt * g_ld);
+        }
+      }
+      // arrives for this lane when its copies so far have landed
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s])) : "memory");
+    }
+    cp_wait<0>();
+    return;
+  }
+
+  const int sub = tid & (DR_LANES - 1), col = blockIdx.x * DR_COLS + tid / DR_LANES;
+  const bool col_ok = col < a.vd;
+  auto piece = [&](int j) { return sub * R + j * 4; };       // first row of this lane's j-th piece
+  float* st = a.state + (((size_t)a.slots[req] * a.heads + h) * a.vd + col) * a.kd;
+  uint64_t s[R / 2];
+#pragma unroll
+  for (int j = 0; j < R / 4; ++j) {
+    ulonglong2 x = make_ulonglong2(0ull, 0ull);
+    if (col_ok && piece(j) < a.kd) x = *reinterpret_cast<const ulonglong2*>(st + piece(j));
+    s[2 * j] = x.x;
+    s[2 * j + 1] = x.y;
+  }
+  const int v_ld = a.heads * a.vd;
+  // values, decay and step size of token `sub` of a stage, in registers a stage ahead
+  float v_next;
+  float2 gb_next;
+  auto ahead = [&](int tb) {
+    const int t = tb + sub;
+    v_next = t < t1 && col_ok ? a.v[(size_t)t * v_ld + (size_t)h * a.vd + col] : 0.f;
+    gb_next = t < t1 ? *reinterpret_cast<const float2*>(a.gb + ((size_t)t * a.heads + h) * 2) : make_float2(0.f, 0.f);
+  };
+  ahead(t0);
+  for (int i = 0; i < stages; ++i) {
+    const int tb = t0 + i * DR_TOK, nt = min(DR_TOK, t1 - tb);
+    const float v_now = v_next;
+    const float2 gb_now = gb_next;
+    ahead(tb + DR_TOK);
+    const bool ok = mbar_wait(&full[i % DR_STAGES], (i / DR_STAGES) & 1, abort_flag);
+    if (!__all_sync(0xffffffffu, ok)) {
+      if (lane == 0) { *abort_flag = 1; atomicExch(status, ERR_DR_CONSUMER); }
+      return;
+    }
+    const float* stage = dr_smem + (i % DR_STAGES) * C::STAGE + sub * C::CH;
+    auto fetch = [&](int array, int tt, uint64_t* to) {
+#pragma unroll
+      for (int j = 0; j < R / 4; ++j) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(stage + (array * DR_TOK + tt) * C::ROW + j * 4);
+        to[2 * j] = x.x;
+        to[2 * j + 1] = x.y;
+      }
+    };
+    uint64_t kn[R / 2], qn[R / 2];
+    fetch(0, 0, kn);
+    fetch(1, 0, qn);
+    auto token = [&](int tt, bool more, float (&xb)[DR_TOK], float (&xc)[DR_TOK], float& u_mine) {
+      uint64_t kr[R / 2], qr[R / 2];
+#pragma unroll
+      for (int j = 0; j < R / 2; ++j) { kr[j] = kn[j]; qr[j] = qn[j]; }
+      if (more) { fetch(0, tt + 1, kn); fetch(1, tt + 1, qn); }   // the next token's parts are on their way during this token's sums
+      if (MODE == 2) {   // the rows decay first, each by its own factor; the sums below then see the decayed state
+        uint64_t d[R / 2];
+        fetch(2, tt, d);
+#pragma unroll
+        for (int j = 0; j < R / 2; ++j) s[j] = mul2(s[j], d[j]);
+      }
+      // four partial sums each: short chains of dependent operations
+      uint64_t pa[2] = {0ull, 0ull}, pb[2] = {0ull, 0ull}, pc[2] = {0ull, 0ull};
+#pragma unroll
+      for (int j = 0; j < R / 2; ++j) {
+        if (MODE != 1) pa[j & 1] = fma2(s[j], kr[j], pa[j & 1]);
+        pb[j & 1] = fma2(s[j], qr[j], pb[j & 1]);
+        pc[j & 1] = fma2(kr[j], qr[j], pc[j & 1]);
+      }
+      auto joined = [](const uint64_t* p) {
+        const float2 x = halves_of(p[0]), y = halves_of(p[1]);
+        return (x.x + x.y) + (y.x + y.y);
+      };
+      // what the state's next value needs is summed over the group at once, the read-out at the end of the stage
+      xc[tt] = joined(pc);
+      xb[tt] = joined(pb);
+      float xa = MODE != 1 ? joined(pa) : 0.f;
+      if (MODE != 1) {
+#pragma unroll
+        for (int o = DR_LANES / 2; o > 0; o >>= 1) xa += __shfl_xor_sync(0xffffffffu, xa, o);
+      }
+      const int from = (lane & ~(DR_LANES - 1)) | tt;
+      const float g = __shfl_sync(0xffffffffu, gb_now.x, from);   // mode 2: g = 1, the rows have decayed already
+      const float beta = MODE == 1 ? 0.f : __shfl_sync(0xffffffffu, gb_now.y, from);
+      const uint64_t gg = pair_of(g, g);
+      float u;
+      if (MODE == 1) {
+        u = __shfl_sync(0xffffffffu, u_mine, from);
+      } else {
+        u = __fmul_rn(beta, fmaf(-g, xa, __shfl_sync(0xffffffffu, v_now, from)));
+        if (sub == tt) u_mine = u;
+      }
+      const uint64_t uu = pair_of(u, u);
+#pragma unroll
+      for (int j = 0; j < R / 2; ++j) s[j] = fma2(kr[j], uu, mul2(gg, s[j]));
+    };
+    float xb[DR_TOK], xc[DR_TOK], u_mine = MODE == 1 ? __fmul_rn(gb_now.y, v_now) : 0.f;   // u_mine: of token `sub`
+    if (nt == DR_TOK) {   // a whole stage without branches, so that loads of later tokens can move ahead of earlier sums
+#pragma unroll
+      for (int tt = 0; tt < DR_TOK; ++tt) token(tt, tt + 1 < DR_TOK, xb, xc, u_mine);
+    } else {
+#pragma unroll
+      for (int tt = 0; tt < DR_TOK; ++tt) {
+        xb[tt] = xc[tt] = 0.f;
+        if (tt < nt) token(tt, tt + 1 < nt, xb, xc, u_mine);
+      }
+    }
+    const float kq = sum_per_token(xc, sub);
+    const float o = fmaf(u_mine, kq, __fmul_rn(gb_now.x, sum_per_token(xb, sub)));
+    if (sub < nt && col_ok) a.out[(size_t)(tb + sub) * v_ld + (size_t)h * a.vd + col] = o;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[i % DR_STAGES]);
+  }
+#pragma unroll
+  for (int j = 0; j < R / 4; ++j)
+    if (col_ok && piece(j) < a.kd) *reinterpret_cast<ulonglong2*>(st + piece(j)) = make_ulonglong2(s[2 * j], s[2 * j + 1]);
+}
+
+template <int R, int MODE>
+static int launch_stream(const ScanArgs& a, dim3 grid, int* status, cudaStream_t s) {
+  using C = Stream<R, MODE>;
+  auto kern = delta_rule_stream_kernel<R, MODE>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "delta_rule_scan: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
+    configured = true;
+  }
+  TLLM_LAUNCH("delta_rule_scan", kern, grid, C::WARPS * 32 + 32, C::SMEM, s, a, status);
+  return TLLM_OK;
+}
+
 // gated_group_norm: y = (o + D_h x) * silu(z), then y / sqrt(mean(y^2) + eps) * w over each of `parts` equal parts of a
 // token's row (a part need not be a head), in 32-bit; one CTA per (token, part).  o, x float32 [T, width] (x and D
 // may be absent), z rows of ldz values in the engine's dtype, w float32 [width], out [T, width] in the engine's dtype.
@@ -422,7 +654,7 @@ extern "C" int tllm_conv_state_update(const void* proj, int ld, float* kept, con
 
 extern "C" int tllm_delta_rule_scan(const float* q, const float* k, const float* v, const float* gb, float* state,
                                     const int* slots, const int* cu_q, float* out, int heads, int kv_heads, int kd, int vd,
-                                    int n_requests, int mode, const float* gk, void* stream) {
+                                    int n_requests, int mode, const float* gk, int* status, void* stream) {
   TLLM_REQUIRE(n_requests > 0 && n_requests <= 65535 && heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0,
                "delta_rule_scan: %d requests, %d heads over %d query/key heads", n_requests, heads, kv_heads);
   TLLM_REQUIRE(kd >= 1 && kd <= 256 && vd >= 1, "delta_rule_scan: key size %d (at most 256), value size %d", kd, vd);
@@ -432,6 +664,20 @@ extern "C" int tllm_delta_rule_scan(const float* q, const float* k, const float*
   TLLM_REQUIRE(mode >= 0 && mode <= 2 && (mode == 2) == (gk != nullptr), "delta_rule_scan: mode %d (0, 1 or 2; decays per key channel with 2 only)", mode);
   const dim3 grid((vd + DR_COLS - 1) / DR_COLS, heads, n_requests);
   cudaStream_t s = (cudaStream_t)stream;
+  // key rows, decays and state columns of whole 16-byte pieces: the streamed kernel
+  if ((kd & 3) == 0 && status != nullptr && (((size_t)q | (size_t)k | (size_t)gk | (size_t)state) & 15) == 0 && ((size_t)gb & 7) == 0) {
+#define TLLM_STREAM(R)                                                            \
+  do {                                                                            \
+    if (mode == 0) return launch_stream<R, 0>(a, grid, status, s);                \
+    if (mode == 1) return launch_stream<R, 1>(a, grid, status, s);                \
+    return launch_stream<R, 2>(a, grid, status, s);                               \
+  } while (0)
+    if (kd <= 32) TLLM_STREAM(4);
+    if (kd <= 64) TLLM_STREAM(8);
+    if (kd <= 128) TLLM_STREAM(16);
+    TLLM_STREAM(32);
+#undef TLLM_STREAM
+  }
 #define TLLM_SCAN(R)                                                                                         \
   do {                                                                                                       \
     if (mode == 0) TLLM_LAUNCH("delta_rule_scan", (delta_rule_scan_kernel<R, 0>), grid, 128, 0, s, a);       \

@@ -24,7 +24,7 @@ BASE_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-shared", "-Xcompiler", "-fPIC"
 HEADERS = ["common.cuh"]
 EXTRA_HEADERS = {"sampling": ["sampling_noalloc.h"], "attention_mma": ["attention_tiles.cuh"],
                  "attention_maps_mma": ["attention_tiles.cuh"], "attention_talk_mma": ["attention_tiles.cuh"],
-                 "linear_tc": ["tc_common.cuh"], "linear_generic": ["tc_common.cuh"],
+                 "linear_tc": ["tc_common.cuh"], "linear_generic": ["tc_common.cuh"], "delta_rule": ["tc_common.cuh"],
                  "attention_tc": ["tc_common.cuh"],
                  "window_attention": ["window_attention.cuh"], "window_attention_mma": ["window_attention.cuh"]}   # per-source headers that enter the hash
 
