@@ -2,7 +2,12 @@
 (main.cpp:10-18) and of Pipeline::apply (tiny_llm/pipeline/pipeline.cpp:100-103, 156-164)."""
 from __future__ import annotations
 
+import struct
+
 from dataclasses import dataclass
+
+# what the device needs of a row's options: temperature (0: greedy), top_p, top_k, seed
+ROW = struct.Struct("=ddiq")
 
 
 @dataclass(frozen=True)
@@ -24,3 +29,8 @@ class SamplingParams:
             raise ValueError("top_k must not be negative")
         if not 0.0 <= self.top_p <= 1.0:
             raise ValueError("top_p must lie in [0, 1]")
+        try:      # packed once per request, not once per token (options of other types are converted by the sampler)
+            row = ROW.pack(self.temperature if self.do_sample else 0.0, self.top_p, self.top_k, self.seed & 0x7FFFFFFFFFFFFFFF)
+        except (struct.error, TypeError, OverflowError):
+            row = None
+        object.__setattr__(self, "packed", row)

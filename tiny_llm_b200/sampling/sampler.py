@@ -10,6 +10,8 @@ import torch
 from .. import ops
 from .params import SamplingParams
 
+_ROW = np.dtype([("temperature", "f8"), ("top_p", "f8"), ("top_k", "i4"), ("seed", "i8")])   # params.ROW
+
 
 def uniform_from(seed: int, counter: int) -> float:
     """The uniform number in [0, 1) the sampling kernel draws for (seed, counter): splitmix64 of
@@ -41,6 +43,8 @@ class Sampler:
         # one host block: temperature f32 | top_p f32 | top_k i32 | seeds i64 | counters i64, as int32 words
         self._words = self.max_rows * 7
         self._host = [torch.zeros(self._words, dtype=torch.int32, pin_memory=pin) for _ in range(self.RING)]
+        self._host_regions = [[x.numpy() for x in self._views(h, self.max_rows)] for h in self._host]
+        self._dev_views = None
         self._host_free = [None] * self.RING      # event: the copy that last read this block has run
         self._dev = torch.zeros(self._words, dtype=torch.int32, device=self.device)
         # the chosen ids, and behind them the status word of the step's kernels (see collect)
@@ -54,6 +58,20 @@ class Sampler:
         m = self.max_rows
         return (buf[0:n].view(torch.float32), buf[m:m + n].view(torch.float32), buf[2 * m:2 * m + n],
                 buf[3 * m:3 * m + 2 * n].view(torch.int64), buf[5 * m:5 * m + 2 * n].view(torch.int64))
+
+    @staticmethod
+    def _fill(regions, n, params, counters) -> None:
+        t, pp, k, s, c = regions
+        try:
+            rows = np.frombuffer(b"".join([p.packed for p in params]), dtype=_ROW)
+        except (AttributeError, TypeError):      # options that do not pack: converted one by one
+            t[:n] = [p.temperature if p.do_sample else 0.0 for p in params]
+            pp[:n] = [p.top_p for p in params]
+            k[:n] = [p.top_k for p in params]
+            s[:n] = np.array([p.seed & 0x7FFFFFFFFFFFFFFF for p in params], dtype=np.int64)
+        else:
+            t[:n], pp[:n], k[:n], s[:n] = rows["temperature"], rows["top_p"], rows["top_k"], rows["seed"]
+        c[:n] = np.array(list(counters), dtype=np.int64)
 
     def launch(self, logits: torch.Tensor, params: Sequence[SamplingParams], counters: Sequence[int]) -> SampleTicket:
         """Enqueues the choice of one token per row of `logits` and its copy to the host;
@@ -70,12 +88,7 @@ class Sampler:
             if self._host_free[slot] is not None:
                 self._host_free[slot].synchronize()
             host = self._host[slot]
-            t, pp, k, s, c = self._views(host, n)
-            t.numpy()[:] = [p.temperature if p.do_sample else 0.0 for p in params]
-            pp.numpy()[:] = [p.top_p for p in params]
-            k.numpy()[:] = [p.top_k for p in params]
-            s.numpy()[:] = np.array([p.seed & 0x7FFFFFFFFFFFFFFF for p in params], dtype=np.int64)
-            c.numpy()[:] = np.array(list(counters), dtype=np.int64)
+            self._fill(self._host_regions[slot], n, params, counters)
             self._dev.copy_(host, non_blocking=True)
             if self.device.type == "cuda":
                 if self._host_free[slot] is None:
@@ -83,7 +96,9 @@ class Sampler:
                 self._host_free[slot].record()
             if self._work is None or self._work.numel() < n * self.vocab_size:
                 self._work = torch.empty(max(n, 8) * self.vocab_size, dtype=torch.float32, device=self.device)
-            dt, dpp, dk, ds, dc = self._views(self._dev, n)
+            if self._dev_views is None or self._dev_views[0] != n:      # the views of the last number of rows
+                self._dev_views = (n, self._views(self._dev, n))
+            dt, dpp, dk, ds, dc = self._dev_views[1]
             ops.sample(logits, self._work, dt, dk, dpp, ds, dc, out, self._status)
         self._out_host[slot][:n + 1].copy_(out, non_blocking=True)
         event = None
