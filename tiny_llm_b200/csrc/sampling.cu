@@ -2,9 +2,10 @@
 //   argmax: first maximum, lowest index on ties (tiny_llm/logit_processors/argmax_processor.cpp:24-31).
 //   sample: the reference's chain temperature -> top-k -> top-p -> multinomial
 //     (tiny_llm/pipeline/pipeline.cpp:157-161), which it runs on the CPU with sorts
-//     (sort_processors.cpp:53-142, sample_processors.cpp:7-54).  Here nothing is sorted: the k-th
-//     largest value and the top-p cut are found by a bitwise search over the ordered bit patterns
-//     of the values, each probe being one counting pass over the row.
+//     (sort_processors.cpp:53-142, sample_processors.cpp:7-54).  Here rows of up to 32,768 stay in
+//     registers and only the few values that survive a bound are ranked (sample_row_kernel); in
+//     longer rows the k-th largest value and the top-p cut are found by a bitwise search over the
+//     ordered bit patterns of the values, each probe being one counting pass over the row.
 //       top-k keeps exactly k values: those above the k-th largest, and of those equal to it the
 //         ones with the lowest token ids.
 //       top-p drops the smallest values while their summed probability stays <= 1 - p; values
@@ -13,7 +14,7 @@
 //         probability exceeds u, u in [0,1) drawn from (seed, counter) of the row by splitmix64, so a
 //         request's draws do not depend on its batch.
 //     A row with temperature <= 0 is taken greedily.
-// `work` is scratch of n*V floats in global memory: the row's scaled logits, then its weights.
+// `work` is scratch of n*V floats in global memory: the row's scaled logits, then its weights (rows that are walked there).
 #include <math_constants.h>
 
 #include "common.cuh"

@@ -1331,8 +1331,8 @@ def fused_qkv_preferred(m: int, n: int, k: int) -> bool:
     return m <= qkv_fused_rows or m > 128 or _cluster_slices(n, k) < 8
 
 
-# float32 products of at most 16 rows take a kernel of their own (one thread per output element, weights streamed
-# through shared memory); False keeps the 64 x 64 tiles.  Both give the same bits (tests compare them).
+# float32 products whose rows start on 16 bytes take the streaming kernel (at most 16 rows) or tiles chosen by size;
+# False keeps the 64 x 64 tiles for all.  All give the same bits (tests compare them).
 linear_skinny = True
 
 
