@@ -1,0 +1,64 @@
+"""What the CUDA sources' host side promises, checked without a GPU."""
+import glob
+import os
+import re
+import shutil
+import subprocess
+
+import pytest
+
+from tiny_llm_b200.ops import build
+
+
+def sources():
+    return {os.path.basename(f): open(f).read()
+            for f in sorted(glob.glob(os.path.join(build.CSRC, "*.cu")) + glob.glob(os.path.join(build.CSRC, "*.cuh")))}
+
+
+PER_DEVICE = r"""
+#include <thread>
+#include <vector>
+#include "per_device.h"
+#define CHECK(x) do { if (!(x)) return __LINE__; } while (0)
+int main() {
+  static tllm::PerDeviceLimit limit;
+  int calls = 0;
+  auto fine = [&] { ++calls; return 0; };
+  for (int dev = 0; dev < 4; ++dev) {               // every ordinal is set up, once
+    for (int i = 0; i < 3; ++i) CHECK(limit.raise(dev, 100, fine) == 0);
+    CHECK(calls == dev + 1);
+  }
+  calls = 0;
+  CHECK(limit.raise(2, 60, fine) == 0 && calls == 0);       // less than what is set
+  CHECK(limit.raise(2, 200, fine) == 0 && calls == 1);      // more, on this device alone
+  CHECK(limit.raise(3, 100, fine) == 0 && calls == 1);
+  CHECK(limit.raise(5, 100, [] { return 7; }) == 7);        // a failure is handed on and tried again
+  CHECK(limit.raise(5, 100, fine) == 0 && calls == 2);
+  for (int dev : {-1, tllm::PerDeviceLimit::DEVICES}) {     // no place for these: set at every call
+    CHECK(limit.raise(dev, 1, fine) == 0 && limit.raise(dev, 1, fine) == 0);
+  }
+  CHECK(calls == 6);
+  std::atomic<int> at_once{0};
+  std::vector<std::thread> threads;
+  for (int i = 0; i < 8; ++i)
+    threads.emplace_back([&] { for (int dev = 8; dev < 40; ++dev) limit.raise(dev, 10, [&] { ++at_once; return 0; }); });
+  for (auto& t : threads) t.join();
+  CHECK(at_once == 32);
+  return 0;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_a_limit_is_raised_once_on_every_device(tmp_path):
+    src, exe = tmp_path / "per_device.cpp", tmp_path / "per_device"
+    src.write_text(PER_DEVICE)
+    res = subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", build.CSRC, "-o", str(exe), str(src)], capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr
+    assert subprocess.run([str(exe)], timeout=60).returncode == 0      # else the line of the check
+
+
+def test_every_launch_raises_its_shared_memory_per_device():
+    """cudaFuncSetAttribute holds for the current device only: it is called in one place, which keeps a limit per device."""
+    where = {name: text.count("cudaFuncSetAttribute(") for name, text in sources().items()}
+    assert {n: c for n, c in where.items() if c} == {"common.cuh": 1}

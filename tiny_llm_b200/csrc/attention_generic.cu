@@ -662,12 +662,7 @@ static int launch_rows(const float* q, int q_row_stride, const float* kcache, co
                        int max_blocks, const int* token_request, const int* positions, float* out, int n_tokens,
                        const Geometry& g, float scale, const float* sink, long long blocks, cudaStream_t s) {
   auto kern = paged_attention_rows_kernel<OD, R>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RowsSmem<OD, R>::BYTES);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "attention: cannot reserve %d bytes of shared memory: %s", RowsSmem<OD, R>::BYTES, cudaGetErrorString(e));
-    configured = true;
-  }
+  TLLM_RESERVE_SMEM("attention", (RowsSmem<OD, R>::BYTES), kern);
   TLLM_LAUNCH("paged_attention_rows", kern, (unsigned)blocks, WAYS * 32, (RowsSmem<OD, R>::BYTES), s, q, q_row_stride, kcache, vcache,
               block_table, max_blocks, token_request, positions, out, n_tokens, g, scale, sink);
   return TLLM_OK;

@@ -438,13 +438,7 @@ extern "C" int tllm_attention_maps_mma(const void* q, int q_row_stride, const vo
   TLLM_REQUIRE(gx <= 2147483647LL, "attention_maps_mma: grid too large");
   constexpr int ST = 2;
   const int smem = (BM * LDK + ST * BN * (LDK + LDV)) * 2 + TABLE_SLOTS * 4;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_maps_kernel<ST, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_maps_kernel<ST, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "attention_maps_mma: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    configured = true;
-  }
+  TLLM_RESERVE_SMEM("attention_maps_mma", smem, (attention_maps_kernel<ST, false>), (attention_maps_kernel<ST, true>));
   const dim3 grid((unsigned)gx, (unsigned)splits);
   if (rel != nullptr) TLLM_LAUNCH("attention_maps_mma", (attention_maps_kernel<ST, true>), grid, 128, smem, (cudaStream_t)stream, p);
   else TLLM_LAUNCH("attention_maps_mma", (attention_maps_kernel<ST, false>), grid, 128, smem, (cudaStream_t)stream, p);

@@ -338,13 +338,7 @@ extern "C" int tllm_attention_mma(const void* q, int q_row_stride, const void* k
     TLLM_REQUIRE(small && tllm_attention_mma_wide_fits() && max_kv_len > 0 && ((max_kv_len + BN - 1) / BN + splits - 1) / splits <= 4,
                  "attention_mma: one warp per tile needs decoded tokens and slices of at most four tiles (%d keys in %d slices)",
                  max_kv_len, splits);
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(attention_decode_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, WIDE_SMEM);
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, WIDE_SMEM);
-      if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "attention_mma: cannot reserve %d bytes of shared memory: %s", WIDE_SMEM, cudaGetErrorString(e));
-      configured = true;
-    }
+    TLLM_RESERVE_SMEM("attention_mma", WIDE_SMEM, attention_decode_wide_kernel<false>, attention_decode_wide_kernel<true>);
     if (cluster) {
       cudaError_t e = launch_z_clusters(attention_decode_wide_kernel<true>, dim3((unsigned)n_requests, nkv, splits), WIDE_SMEM, s, p);
       if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "attention_decode_wide (cluster of %d): %s", splits, cudaGetErrorString(e));
@@ -356,22 +350,12 @@ extern "C" int tllm_attention_mma(const void* q, int q_row_stride, const void* k
     // the merge buffers (4 x 16 x (HD + 2) floats) reuse the tile stages
     static_assert(4 * 16 * (HD + 2) * 4 <= ST * BN * LDS * 2, "merge buffers must fit the key stages");
     const int smem = (16 + 2 * ST * BN) * LDS * 2 + TABLE_SLOTS * 4;
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "attention_mma: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-      configured = true;
-    }
+    TLLM_RESERVE_SMEM("attention_mma", smem, attention_decode_kernel<ST>);
     TLLM_LAUNCH("attention_decode", attention_decode_kernel<ST>, dim3((unsigned)n_requests, nkv, splits), 128, smem, s, p);
   } else {
     constexpr int ST = 2;
     const int smem = (64 + 2 * ST * BN) * LDS * 2 + TABLE_SLOTS * 4;
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(attention_mma_kernel<4, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "attention_mma: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
-      configured = true;
-    }
+    TLLM_RESERVE_SMEM("attention_mma", smem, (attention_mma_kernel<4, ST>));
     TLLM_REQUIRE(gx * nkv <= 2147483647LL, "attention_mma: grid too large");
     TLLM_LAUNCH("attention_mma", (attention_mma_kernel<4, ST>), dim3((unsigned)(gx * nkv), 1, splits), 128, smem, s, p);
   }

@@ -453,12 +453,7 @@ static int launch_conv(const ConvArgs& a, cudaStream_t s) {
   const int channels = (a.nq + a.nkv) * a.kd + a.nkv * a.vd, pieces = channels / V;
   const int threads = pieces >= CONV_THREADS ? CONV_THREADS : (pieces + 31) / 32 * 32;
   const size_t smem = (size_t)TOK * ((a.nq + a.nkv) * a.kd + a.rot_dims) * 4;
-  static size_t configured = 48 * 1024;
-  if (smem + 2 * TOK * 33 * 4 > configured) {
-    cudaError_t e = cudaFuncSetAttribute(conv_norm_kv_write_kernel<T, V, TOK, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "conv_norm_kv_write: cannot reserve %d bytes of shared memory: %s", (int)smem, cudaGetErrorString(e));
-    configured = smem + 2 * TOK * 33 * 4;
-  }
+  if (smem + 2 * TOK * 33 * 4 > 48 * 1024) TLLM_RESERVE_SMEM("conv_norm_kv_write", smem, (conv_norm_kv_write_kernel<T, V, TOK, NT>));   // (with its static part)
   TLLM_LAUNCH("conv_norm_kv_write", (conv_norm_kv_write_kernel<T, V, TOK, NT>), (unsigned)((a.n_tokens + TOK - 1) / TOK), threads, smem, s, a);
   return TLLM_OK;
 }

@@ -207,12 +207,7 @@ inline size_t talk_smem(int qt, int TK_KEYS, int heads, int kv_heads, int kd, in
 template <typename T, int QT, int VC>
 int talk_launch(const TalkArgs& a, int n_requests, int max_q_len, size_t smem, cudaStream_t s) {
   auto kernel = attention_talk_kernel<T, QT, VC>;
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      TLLM_FAIL(TLLM_ERR_CUDA, "attention_talk: %zu bytes of shared memory were refused", smem);
-    configured = smem;
-  }
+  if (smem > 48 * 1024) TLLM_RESERVE_SMEM("attention_talk", smem, kernel);
   const dim3 grid((max_q_len + QT - 1) / QT, n_requests);
   TLLM_LAUNCH("attention_talk", kernel, grid, 32 * a.heads, smem, s, a);
   return TLLM_OK;

@@ -390,12 +390,7 @@ extern "C" int tllm_attention_talk_mma(const void* q, int ldq, const void* kcach
   const size_t smem = talk_mma_smem(heads, kv_heads, stages);
   TLLM_REQUIRE(smem <= LIMIT, "attention_talk_mma: %d heads over %d key/value heads of %d / %d values need %zu bytes of shared memory",
                heads, kv_heads, KD, VD, smem);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    if (cudaFuncSetAttribute(attention_talk_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-      TLLM_FAIL(TLLM_ERR_CUDA, "attention_talk_mma: %zu bytes of shared memory were refused", smem);
-    configured = smem;
-  }
+  if (smem > 48 * 1024) TLLM_RESERVE_SMEM("attention_talk_mma", smem, attention_talk_mma_kernel);
   TalkMmaArgs a;
   a.q = (const __nv_bfloat16*)q; a.ldq = ldq; a.kcache = (const __nv_bfloat16*)kcache; a.vcache = (const __nv_bfloat16*)vcache;
   a.block_table = block_table; a.max_blocks = max_blocks; a.cu_q = cu_q; a.q_start = q_start; a.mix = mix_log2; a.sink = sink;

@@ -562,12 +562,7 @@ extern "C" int tllm_attention_tc(const void* q, int q_row_stride, const void* kc
   p.scale_log2 = scale * 1.4426950408889634f;
   const long long gx = (long long)n_requests * p.tiles_per_req * nkv;
   TLLM_REQUIRE(gx <= 2147483647LL, "attention_tc: grid too large");
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "attention_tc: cannot reserve %d bytes of shared memory: %s", SMEM_TOTAL, cudaGetErrorString(e));
-    configured = true;
-  }
+  TLLM_RESERVE_SMEM("attention_tc", SMEM_TOTAL, attention_tc_kernel);
   TLLM_LAUNCH("attention_tc", attention_tc_kernel, dim3((unsigned)gx), THREADS, SMEM_TOTAL, (cudaStream_t)stream, mq, mk, mv, p);
   return TLLM_OK;
 }

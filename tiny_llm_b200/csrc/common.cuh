@@ -7,6 +7,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include "per_device.h"
+
 #define TLLM_F32 0
 #define TLLM_BF16 1
 
@@ -161,7 +163,31 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Raises the limit of the kernels' dynamic shared memory to `bytes` on the current device where it is lower; `limit` is one
+// object for these kernels (TLLM_RESERVE_SMEM).
+template <typename... Kernels>
+inline cudaError_t reserve_smem(PerDeviceLimit& limit, long long bytes, Kernels... kernels) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  return (cudaError_t)limit.raise(dev, bytes, [&] {
+    cudaError_t r = cudaSuccess;
+    (void)((r = cudaFuncSetAttribute(kernels, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), r == cudaSuccess) && ...);
+    return (int)r;
+  });
+}
+
 }  // namespace tllm
+
+// Before a launch of `kernels` with more than 48 KB of shared memory: once per device and place in the source.
+#define TLLM_RESERVE_SMEM(name, bytes, ...)                                                                     \
+  do {                                                                                                          \
+    static ::tllm::PerDeviceLimit limit_;                                                                       \
+    cudaError_t e_ = ::tllm::reserve_smem(limit_, (long long)(bytes), __VA_ARGS__);                             \
+    if (e_ != cudaSuccess)                                                                                      \
+      TLLM_FAIL(TLLM_ERR_CUDA, "%s: cannot reserve %lld bytes of shared memory: %s", name, (long long)(bytes),  \
+                cudaGetErrorString(e_));                                                                        \
+  } while (0)
 
 // Each shared object exports its own tllm_last_error() and tllm_set_pdl().
 #ifdef TLLM_TRACE

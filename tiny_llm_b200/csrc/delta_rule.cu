@@ -549,12 +549,7 @@ template <int R, int MODE>
 static int launch_stream(const ScanArgs& a, dim3 grid, int* status, cudaStream_t s) {
   using C = Stream<R, MODE>;
   auto kern = delta_rule_stream_kernel<R, MODE>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "delta_rule_scan: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
-    configured = true;
-  }
+  TLLM_RESERVE_SMEM("delta_rule_scan", C::SMEM, kern);
   TLLM_LAUNCH("delta_rule_scan", kern, grid, C::WARPS * 32 + 32, C::SMEM, s, a, status);
   return TLLM_OK;
 }

@@ -250,12 +250,7 @@ static int launch_tile_mode(const float* a, const float* w, float* out, int m, i
   using C = Tile<WM, WN, TM, TN>;
   auto kern = linear_tiled_kernel<WM, WN, TM, TN, MODE>;
   constexpr int MOST = C::SMEM > C::SMEM_ALONE ? C::SMEM : C::SMEM_ALONE;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "linear_tiled: cannot reserve %d bytes of shared memory: %s", MOST, cudaGetErrorString(e));
-    configured = true;
-  }
+  TLLM_RESERVE_SMEM("linear_tiled", MOST, kern);
   dim3 grid((m + C::M - 1) / C::M, (n + C::N - 1) / C::N);
   // As many CTAs as SMs or fewer: one per SM.  Two that may share an SM do so while others idle (128 CTAs of 64 x 128
   // took 155 us instead of 102).
@@ -452,13 +447,7 @@ static bool make_skinny_map(CUtensorMap* map, const float* ptr, int rows, int k,
 template <int R, int RW, int TR, int W, int KB, int ST>
 int launch_skinny(const float* a, const float* w, float* out, int m, int n, int k, int lda, int ldo, int mode, int* status, cudaStream_t s) {
   using C = Skinny<R, RW, TR, W, KB, ST>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(linear_skinny_kernel<R, RW, TR, W, KB, ST, OUT_ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_skinny_kernel<R, RW, TR, W, KB, ST, OUT_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "linear_skinny: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
-    configured = true;
-  }
+  TLLM_RESERVE_SMEM("linear_skinny", C::SMEM, (linear_skinny_kernel<R, RW, TR, W, KB, ST, OUT_ACC>), (linear_skinny_kernel<R, RW, TR, W, KB, ST, OUT_F32>));
   CUtensorMap mw, ma;
   if (!make_skinny_map(&mw, w, n, k, k, C::ROWS) || !make_skinny_map(&ma, a, m, k, lda, R))
     TLLM_FAIL(TLLM_ERR_CUDA, "linear_skinny: cuTensorMapEncodeTiled failed");

@@ -1011,12 +1011,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, void* out, int r
                   int ldo, int* status, cudaStream_t s) {
   using L = SmemLayout<BN, STAGES>;
   auto kern = linear_tc_kernel<BN, STAGES, SWAP, EPI>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "linear_tc: cannot reserve %d bytes of shared memory: %s", L::TOTAL, cudaGetErrorString(e));
-    configured = true;
-  }
+  TLLM_RESERVE_SMEM("linear_tc", L::TOTAL, kern);
   const int k_blocks = (k + BK - 1) / BK;
   const int per_split = (k_blocks + splits - 1) / splits;
   const int used_splits = (k_blocks + per_split - 1) / per_split;
@@ -1030,16 +1025,10 @@ static int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, void*
                              int* status, cudaStream_t s, const ClusterArgs& ca = ClusterArgs(), const void* w_ptr = nullptr) {
   using L = PersistentSmem<BN, STAGES>;
   auto kern = linear_tc_persistent_kernel<BN, STAGES, EPI>;
-  static bool configured = false;
-  static int sm_count = 0;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "linear_tc: cannot reserve %d bytes of shared memory: %s", L::TOTAL, cudaGetErrorString(e));
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-    configured = true;
-  }
+  TLLM_RESERVE_SMEM("linear_tc", L::TOTAL, kern);
+  int dev = 0, sm_count = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count < 1)
+    TLLM_FAIL(TLLM_ERR_CUDA, "linear_tc: cannot read the number of SMs");
   const int tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
   ClusterArgs args = ca;
   args.tail_from = tiles;
@@ -1095,12 +1084,7 @@ static int launch_cluster(const CUtensorMap& ma, const CUtensorMap& mb, void* ou
                           const ClusterArgs& ca, int* status, cudaStream_t s) {
   using L = SmemLayout<BN, STAGES>;
   auto kern = linear_tc_cluster_kernel<BN, STAGES, EPI>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "linear_tc: cannot reserve %d bytes of shared memory: %s", L::TOTAL, cudaGetErrorString(e));
-    configured = true;
-  }
+  TLLM_RESERVE_SMEM("linear_tc", L::TOTAL, kern);
   const int k_blocks = (k + BK - 1) / BK;
   const int per_split = (k_blocks + ca.cz - 1) / ca.cz;
   const int row_tiles = (rows_a + BM - 1) / BM;

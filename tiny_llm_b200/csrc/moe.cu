@@ -566,12 +566,7 @@ extern "C" int tllm_moe_linear(const void* in, int ld_in, const void* w, const i
 #define TLLM_MOE_MMA(TO, BM, G)                                                                                           \
   do {                                                                                                                    \
     const size_t smem = sizeof(__nv_bfloat16) * (BM == 16 ? 4 : 3) * (BM + 128) * 40 + BM * sizeof(int);                   \
-    static bool configured = false;                                                                                       \
-    if (!configured) {                                                                                                    \
-      cudaError_t e_ = cudaFuncSetAttribute(moe_linear_mma_kernel<TO, BM, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      if (e_ != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "moe_linear: %s", cudaGetErrorString(e_));                           \
-      configured = true;                                                                                                  \
-    }                                                                                                                     \
+    TLLM_RESERVE_SMEM("moe_linear", smem, (moe_linear_mma_kernel<TO, BM, G>));                                            \
     TLLM_LAUNCH("moe_linear", (moe_linear_mma_kernel<TO, BM, G>), grid, 256, smem, s, (const __nv_bfloat16*)in, ld_in,     \
                 (const __nv_bfloat16*)w, sorted_rows, tile_expert, (TO*)out, n, k, rows_per_input, glu_block);             \
   } while (0)

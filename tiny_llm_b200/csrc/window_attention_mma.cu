@@ -297,12 +297,7 @@ extern "C" int tllm_window_pool_attention_mma(const WinArgs* args, const int* cu
   TLLM_REQUIRE(a.row_stride % 8 == 0 && ((uintptr_t)a.qkv & 15) == 0, "window_pool_attention_mma: query rows must be 16-byte aligned");
   TLLM_REQUIRE(a.nkv <= 65535 && n_requests <= 65535, "window_pool_attention_mma: the grid is too large");
   const size_t smem = (size_t)(BM * LDK + 2 * BN * LDK + 2 * BN * LDV) * sizeof(__nv_bfloat16) + 2 * BN * sizeof(int);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(window_pool_attention_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) TLLM_FAIL(TLLM_ERR_CUDA, "window_pool_attention_mma: %s", cudaGetErrorString(e));
-    configured = true;
-  }
+  TLLM_RESERVE_SMEM("window_pool_attention_mma", smem, window_pool_attention_mma_kernel);
   const int tokens_per_tile = BM / G;
   TLLM_REQUIRE(splits >= 1 && (splits == 1 || acc != nullptr), "window_pool_attention_mma: key runs need a float32 buffer");
   const dim3 grid((unsigned)((max_q_len + tokens_per_tile - 1) / tokens_per_tile * splits), (unsigned)a.nkv, (unsigned)n_requests);

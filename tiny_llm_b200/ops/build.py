@@ -21,7 +21,7 @@ from typing import Dict, Optional
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc")
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 BASE_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-shared", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
-HEADERS = ["common.cuh"]
+HEADERS = ["common.cuh", "per_device.h"]
 EXTRA_HEADERS = {"sampling": ["sampling_noalloc.h"], "attention_mma": ["attention_tiles.cuh"],
                  "attention_maps_mma": ["attention_tiles.cuh"], "attention_talk_mma": ["attention_tiles.cuh"],
                  "linear_tc": ["tc_common.cuh"], "linear_generic": ["tc_common.cuh"], "delta_rule": ["tc_common.cuh"],
