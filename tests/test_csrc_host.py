@@ -62,3 +62,22 @@ def test_every_launch_raises_its_shared_memory_per_device():
     """cudaFuncSetAttribute holds for the current device only: it is called in one place, which keeps a limit per device."""
     where = {name: text.count("cudaFuncSetAttribute(") for name, text in sources().items()}
     assert {n: c for n, c in where.items() if c} == {"common.cuh": 1}
+
+
+def test_every_wait_that_gives_up_has_a_code_and_words_of_its_own():
+    from tiny_llm_b200 import ops
+    codes, reports = {}, {}
+    for name, text in sources().items():
+        for role, code in re.findall(r"\b(ERR_[A-Z_]+) = (\d+)", text):
+            assert name == "tc_common.cuh", f"{role} of {name}: the codes are kept in one list"
+            codes[role] = int(code)
+        for role in re.findall(r"atomicExch\([^;]*?(\w+)\)", text):
+            reports.setdefault(role, set()).add(name)
+    assert len(set(codes.values())) == len(codes) and 0 not in codes.values()
+    assert set(reports) == set(codes)
+    assert all(len(files) == 1 for files in reports.values())          # no two kernel families share a code
+    assert set(ops._STATUS_CODES) == set(codes.values()) and len(set(ops._STATUS_CODES.values())) == len(codes)
+    with pytest.raises(ops.KernelError, match=rf"code {codes['ERR_DR_CONSUMER']}: .*scan"):
+        ops.raise_status("cuda:63", codes["ERR_DR_CONSUMER"])
+    with pytest.raises(ops.KernelError, match=rf"code {codes['ERR_SK_PRODUCER']}: .*32-bit product"):
+        ops.raise_status("cuda:63", codes["ERR_SK_PRODUCER"])

@@ -72,7 +72,6 @@ constexpr uint32_t TMEM_COLS = 256;                // S of even tiles: columns [
 constexpr uint32_t TMEM_O = 2 * BNK, TMEM_P = HD == 64 ? TMEM_O + HD : 0, TMEM_P_STEP = HD == 64 ? BNK / 2 : BNK;
 static_assert(TMEM_O + HD <= TMEM_COLS && TMEM_P + TMEM_P_STEP + BNK / 2 <= TMEM_COLS, "S, O and P share 256 columns of tensor memory");
 constexpr float RESCALE_STEP = 8.f;
-constexpr int ERR_ATT_PRODUCER = 7, ERR_ATT_MMA = 8, ERR_ATT_SOFTMAX = 9;
 
 struct TcAttnParams {
   const int* block_table;   // [R, max_blocks]

@@ -358,7 +358,7 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-constexpr int DR_STAGES = 4, ERR_DR_PRODUCER = 1, ERR_DR_CONSUMER = 3;
+constexpr int DR_STAGES = 4;
 
 template <int R, int MODE>
 struct Stream {

@@ -305,7 +305,6 @@ __device__ __forceinline__ float4 read_shared4(uint32_t at) {
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
   return v;
 }
-constexpr int ERR_SK_PRODUCER = 1, ERR_SK_CONSUMER = 3;
 
 template <int R, int RW, int TR, int W, int KB, int ST>
 struct Skinny {

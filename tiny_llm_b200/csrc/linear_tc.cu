@@ -45,8 +45,6 @@ enum Epilogue { EPI_BF16 = 0, EPI_F32 = 1, EPI_ADD_F32 = 2, EPI_SWIGLU = 3, EPI_
                 EPI_GLU_CLAMPED = 11,     // like EPI_SWIGLU with the clamped gate (glu_f)
                 EPI_GLU_GELU = 12 };      // like EPI_SWIGLU with the tanh form of GELU (glu_f)
 
-constexpr int ERR_PRODUCER = 1, ERR_MMA = 2, ERR_EPILOGUE = 3;
-
 __device__ __forceinline__ float silu_f(float x) { return __fdividef(x, 1.f + __expf(-x)); }
 
 // What the gate/up epilogues store: SiLU(g) u, or, clamped, with g <- min(g, limit) and u <- clamp(u, -limit, limit),

@@ -1224,8 +1224,13 @@ def status_word(device) -> torch.Tensor:
     return _status[key]
 
 
-_STATUS_CODES = ("1 = TMA producer, 2 = MMA issuer, 3 = epilogue of a matrix product; 7 = TMA producer, "
-                 "8 = MMA issuer, 9 = softmax of the tensor-core attention")
+# what the ERR_ codes of csrc/tc_common.cuh stand for
+_STATUS_CODES = {1: "TMA producer of a tensor-core product", 2: "MMA issuer of a tensor-core product",
+                 3: "epilogue of a tensor-core product",
+                 7: "TMA producer of the tensor-core attention", 8: "MMA issuer of the tensor-core attention",
+                 9: "softmax of the tensor-core attention",
+                 10: "TMA producer of a streamed 32-bit product", 11: "computing warp of a streamed 32-bit product",
+                 12: "copying warp of a delta-rule or state-space scan", 13: "computing warp of a delta-rule or state-space scan"}
 
 
 def raise_status(device, code: int) -> None:
@@ -1233,7 +1238,7 @@ def raise_status(device, code: int) -> None:
     key = torch.device(device).index or 0
     if key in _status:
         _status[key].zero_()
-    raise KernelError(f"a kernel on device {key} gave up waiting (code {code}: {_STATUS_CODES}); "
+    raise KernelError(f"a kernel on device {key} gave up waiting (code {code}: {_STATUS_CODES.get(code, 'unknown')}); "
                       f"the step's output is not valid and was dropped")
 
 
