@@ -326,6 +326,26 @@ def test_float32_tiles_of_every_size_give_the_bits_of_the_tile_kernel(ops, m, n,
     assert float((outs[0][0][:, :n] - ref).abs().max()) <= k * 2.0 ** -23 * float(a.abs().max() * w.abs().max()) * math.sqrt(k)
 
 
+@pytest.mark.parametrize("m,n,k", [(17, 64, 64), (100, 192, 256), (509, 40, 1024)])
+def test_float32_products_of_many_rows_wait_for_weights_that_are_being_written(ops, m, n, k):
+    """`w` is the product of the launch just before, which takes long on a few SMs: the others are free for this one."""
+    g = torch.Generator().manual_seed(m)
+    deep = 16384
+    left, right = torch.randn(n, deep, generator=g).to(DEV), (torch.randn(k, deep, generator=g) * deep ** -0.5).to(DEV)
+    a = torch.randn(m, k, generator=g).to(DEV)
+    want_w = torch.empty(n, k, device=DEV)
+    ops.linear(left, right, want_w)
+    want = torch.empty(m, n, device=DEV)
+    torch.cuda.synchronize()
+    ops.linear(a, want_w, want)
+    for _ in range(3):
+        w, out = torch.full((n, k), math.nan, device=DEV), torch.empty(m, n, device=DEV)
+        torch.cuda.synchronize()
+        ops.linear(left, right, w)
+        ops.linear(a, w, out)
+        assert torch.equal(w, want_w) and torch.equal(out, want)
+
+
 @pytest.mark.parametrize("dtype", DT)
 @pytest.mark.parametrize("window", [None, 300])
 @pytest.mark.parametrize("nq,nkv,hd", [(6, 2, 48), (8, 1, 64), (4, 4, 128), (10, 2, 256)])

@@ -163,9 +163,8 @@ linear_tiled_kernel(const float* __restrict__ a, const float* __restrict__ w, fl
       }
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
-    for (int st = 0; st < TST; ++st) copy_w(st);   // the weights depend on no earlier kernel
-    pdl_wait();
-    for (int st = 0; st < TST; ++st) { copy_a(st); commit(); }
+    pdl_wait();   // before the weights too: with this many rows `w` may be what the launch just before has written
+    for (int st = 0; st < TST; ++st) { copy_w(st); copy_a(st); commit(); }
     for (int st = 0; st < steps; ++st) {
       asm volatile("cp.async.wait_group %0;" ::"n"(TST - 1) : "memory");
       // a producer turns what it copied itself, so its own landed groups are all it has to wait for

@@ -1356,7 +1356,10 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool
     that stores bfloat16 cuts K into slices that meet in a thread-block cluster (every SM streams weights; without
     it such a product has one CTA per 128 output columns, which walks all of K).  bfloat16 products run on the tensor
     cores (tcgen05) when K and the row stride of `a` are multiples of 8; float32 products, and
-    the sizes TMA cannot take, run on the SIMT kernel."""
+    the sizes TMA cannot take, run on the SIMT kernel.
+    `w` is taken for a loaded weight: float32 products of at most 16 rows and the tensor-core products begin to read it
+    while earlier launches of this package still run, so none of those may be writing it.  (float32 products of more
+    rows wait first.)"""
     _need_cuda(a, w, out)
     m, k = a.shape
     n = w.shape[0]
