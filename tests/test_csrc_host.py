@@ -81,3 +81,14 @@ def test_every_wait_that_gives_up_has_a_code_and_words_of_its_own():
         ops.raise_status("cuda:63", codes["ERR_DR_CONSUMER"])
     with pytest.raises(ops.KernelError, match=rf"code {codes['ERR_SK_PRODUCER']}: .*32-bit product"):
         ops.raise_status("cuda:63", codes["ERR_SK_PRODUCER"])
+
+
+# kernels whose copies to shared memory complete on an mbarrier
+STREAMED = ["linear_generic.cu"]
+
+
+@pytest.mark.parametrize("name", STREAMED)
+def test_a_producer_that_gives_up_waits_for_its_copies(name):
+    """Every kernel that arms a barrier with the bytes of a copy ends its producer with the wait for the copies in flight."""
+    kernels = [k for k in sources()[name].split("__global__")[1:] if "mbar_expect_tx(" in k]
+    assert kernels and all("mbar_drain(" in k for k in kernels)

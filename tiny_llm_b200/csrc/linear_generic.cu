@@ -356,11 +356,13 @@ linear_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       for (int c = 0; c < pre; ++c) load_w(c);
       pdl_wait();
       for (int c = 0; c < pre; ++c) load_a(c);
-      for (int c = ST; c < chunks; ++c) {
+      int c = pre;
+      for (; c < chunks; ++c) {
         if (!mbar_wait(&empty[c % ST], ((c / ST) & 1) ^ 1, abort_flag)) { *abort_flag = 1; atomicExch(status, ERR_SK_PRODUCER); break; }
         load_w(c);
         load_a(c);
       }
+      mbar_drain(full, ST, c);
     }
     return;
   }

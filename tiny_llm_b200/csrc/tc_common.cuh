@@ -66,6 +66,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     if (global_timer_ns() - t0 > WAIT_LIMIT_NS) return false;
   }
 }
+// The end of a producer that fills a ring of `stages` (fill i arms full[i % stages]): waits, with a limit of its own, for the
+// last fills of the `issued` ones, so that no copy is in flight when the CTA ends, also where the roles that were to wait
+// for it gave up (the shared memory could be another CTA's by the time they land).  Otherwise it costs nothing: the
+// readers of the last stage end later.
+constexpr unsigned long long DRAIN_LIMIT_NS = 2000000000ull;
+__device__ __forceinline__ void mbar_drain(uint64_t* full, int stages, int issued) {
+  const unsigned long long t0 = global_timer_ns();
+  for (int i = issued > stages ? issued - stages : 0; i < issued; ++i)
+    while (!mbar_try_wait(&full[i % stages], (i / stages) & 1))
+      if (global_timer_ns() - t0 > DRAIN_LIMIT_NS) return;
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
