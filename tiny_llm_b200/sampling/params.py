@@ -10,8 +10,13 @@ from dataclasses import dataclass
 ROW = struct.Struct("=ddiq")
 
 
+class _Packed:
+    """The packed row beside the options: not one of their fields, so not in vars() either."""
+    __slots__ = ("packed",)
+
+
 @dataclass(frozen=True)
-class SamplingParams:
+class SamplingParams(_Packed):
     max_new_tokens: int = 256   # cap on generated tokens
     do_sample: bool = True      # False: greedy (first maximum)
     temperature: float = 0.7    # logits are divided by it
@@ -29,8 +34,18 @@ class SamplingParams:
             raise ValueError("top_k must not be negative")
         if not 0.0 <= self.top_p <= 1.0:
             raise ValueError("top_p must lie in [0, 1]")
-        try:      # packed once per request, not once per token (options of other types are converted by the sampler)
+        self._pack()
+
+    def _pack(self):      # once per request, not once per token (options of other types are converted by the sampler)
+        try:
             row = ROW.pack(self.temperature if self.do_sample else 0.0, self.top_p, self.top_k, self.seed & 0x7FFFFFFFFFFFFFFF)
         except (struct.error, TypeError, OverflowError):
             row = None
         object.__setattr__(self, "packed", row)
+
+    def __getstate__(self):
+        return dict(self.__dict__)
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        self._pack()
