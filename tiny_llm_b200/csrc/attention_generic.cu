@@ -340,9 +340,9 @@ paged_attention_grouped_kernel(const T* __restrict__ q, int q_row_stride, const 
 // for.  Here a tile's keys and values come to shared memory by cp.async (the next tile's while this one is worked on),
 // once for all rows; a lane still is a key for the scores and a value column for the output, and the rows go in pairs
 // through fma.rn.f32x2, whose halves round like fmaf.  The sums over a tile's 32 keys keep the tree of warp_sum: partners
-// exchange halves of the rows instead of whole rows, so R rows take R steps of shuffles instead of 5 R.
-// Bound by the reads of shared memory. us per layer at the TinyLlama sizes, this kernel / the launches above: a prompt of
-// 509 tokens 180 / 381, eight decoded tokens at context 700 30 / 68.
+// exchange halves of the rows instead of whole rows, so 16 rows take 16 steps of shuffles instead of 80 and 4 rows 6
+// instead of 20.  us per layer at the TinyLlama sizes, this kernel / the launches above: a prompt of 509 tokens 110 / 351,
+// eight decoded tokens at context 700 18 / 42.
 __device__ __forceinline__ uint64_t pack_pair(float lo, float hi) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -420,7 +420,8 @@ paged_attention_rows_kernel(const float* __restrict__ q, int q_row_stride, const
   pdl_wait();
   const int kd = g.kd, vd = g.vd, maps = g.maps, page_size = g.page_size;
   const int group = g.nq / g.nk, kh = blockIdx.x % g.nk, vh = kh / maps, map = kh % maps;
-  // later tokens see more keys: their tiles start first
+  // a request's later tokens see more keys: the step's last rows start first (with decoded tokens ahead of a prompt, as the
+  // scheduler lays a step out, those start last)
   const long long first = (long long)(gridDim.x / g.nk - 1 - blockIdx.x / g.nk) * R;
   const long long n_rows = (long long)n_tokens * group;
   const int t_first = (int)(first / group), t_last = (int)((min(first + R, n_rows) - 1) / group);
@@ -468,10 +469,13 @@ paged_attention_rows_kernel(const float* __restrict__ q, int q_row_stride, const
       while (j0 <= p_max && !tile_seen(g, j0, lo_min, p_max)) j0 = next_tile(g, j0, 32 * WAYS, first_group);
       return j0;
     };
-    // this lane's key of the tile at j0: its page, or -1
+    // this lane's key of the tile at j0: its page, or -1.  Every lane looks a page up (the last seen key's where it has no
+    // key): with the lookup behind a branch the lanes with and without a key went through the scores and the softmax of the
+    // tile before one after the other, 14 us on a request whose last tile of several is not whole (us per launch, eight
+    // decoded tokens with 256 / 257 / 700 keys: 8.8 / 25.2 / 31.4, now 8.8 / 12.2 / 18.4)
     auto page_of = [&](int j0) {
-      const int j = j0 + lane;
-      return j <= p_max && j / page_size < max_blocks ? table[j / page_size] : -1;
+      const int j = j0 + lane, block = min(j, p_max) / page_size, page = table[min(block, max_blocks - 1)];
+      return (j <= p_max) & (block < max_blocks) ? page : -1;
     };
     // rows of the tile to shared memory, a row per OD * 8 lanes; keys without a page stay as they are and are not used
     auto fetch = [&](float* dst, int ld, const float* cache, long long page_stride, long long head_offset, int size, int j0, int page) {
