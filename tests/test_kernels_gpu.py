@@ -876,6 +876,40 @@ def test_attention_of_rows_that_share_their_keys_gives_the_bits_of_one_warp_per_
             assert torch.equal(outs[0], other)
 
 
+@pytest.mark.parametrize("vocab", [900, 1030, 8192, 32000, 32768])
+def test_sample_with_lists_that_are_full_and_lists_that_overflow(ops, vocab):
+    """Limits around the most values that are ranked, and rows whose list does not fit: equal values at the k-th largest,
+    above it, and large values side by side in few threads (more of one thread than it lists, with a bound far below the
+    k-th largest).  The same ids as a row filled up beyond the register kernel's length with minus infinity."""
+    g = torch.Generator().manual_seed(vocab)
+    def crowded():      # thread i holds the ids i, i + 1024, ...: the large values lie in the first 40 threads
+        x = torch.randn(vocab, generator=g)
+        at = torch.arange(vocab)
+        x[at % 1024 < 40] += 20
+        return x
+    def levels(many):
+        x = torch.randn(vocab, generator=g)
+        x[torch.randperm(vocab, generator=g)[:many]] = 9.0
+        x[torch.randperm(vocab, generator=g)[:5]] = 11.0
+        return x
+    kinds = [lambda: torch.randn(vocab, generator=g) * 2.5, lambda: (torch.randn(vocab, generator=g) * 2.5).round(), crowded,
+             lambda: levels(30), lambda: levels(600), lambda: -levels(600)]
+    options = [(k, p, kind) for k in (3, 40, 208, 255, 256, 257, 400) for p in (0.3, 0.9, 1.0) for kind in range(len(kinds))]
+    n = len(options)
+    rows = torch.stack([kinds[kind]() for _, _, kind in options])
+    long = torch.full((n, 33000), -math.inf)
+    long[:, :vocab] = rows
+    temps, ks, ps = torch.full((n,), 0.8), torch.tensor([o[0] for o in options], dtype=torch.int32), torch.tensor([o[1] for o in options])
+    seeds, counters = torch.arange(n, dtype=torch.int64) * 17 + 3, torch.arange(n, dtype=torch.int64) % 5
+    got = []
+    for logits in (rows, long):
+        out = torch.empty(n, dtype=torch.int32, device=DEV)
+        ops.sample(logits.to(DEV), torch.empty(logits.numel(), device=DEV), temps.to(DEV), ks.to(DEV), ps.to(DEV), seeds.to(DEV),
+                   counters.to(DEV), out)
+        got.append(out.cpu().tolist())
+    assert got[0] == got[1]
+
+
 @pytest.mark.parametrize("vocab", [1, 331, 1024, 1025, 8192, 8193, 16385, 32000, 32768])
 def test_sample_in_registers_draws_what_the_passes_over_memory_draw(ops, vocab):
     """Rows of up to 32,768 logits are kept in registers, longer ones are walked in memory.  A row filled up to 33,000

@@ -201,8 +201,11 @@ __device__ __forceinline__ float uniform_from(unsigned long long seed, unsigned 
 }
 
 // The choice of one row in passes over its scratch `x` (v floats in global memory), for any length and any limits.
+// FLOOR: at least k values reach the key `floor`.  With many equal values it often is the k-th largest itself, which one pass
+// tells; else the search needs no pass for what lies up to it.
+template <bool FLOOR>
 __device__ __noinline__ void sample_in_memory(const float* __restrict__ row, float* __restrict__ x, int v, float temp, int k,
-                                              float p, float u, int* __restrict__ out, BlockScratch& sc) {
+                                              float p, float u, uint32_t floor, int* __restrict__ out, BlockScratch& sc) {
   __shared__ int s_choice, s_last;
 
   // scaled logits and their maximum
@@ -217,8 +220,15 @@ __device__ __noinline__ void sample_in_memory(const float* __restrict__ row, flo
   // top-k: tau = ordered key of the k-th largest value
   if (k > 0 && k < v) {
     uint32_t tau = 0;
-    for (int bit = 31; bit >= 0; --bit) {
+    int first = 31;
+    if (FLOOR) {
+      int above = 0;
+      for (int i = threadIdx.x; i < v; i += ST) above += ordered_key(x[i]) > floor;
+      if (block_sum_i(above, sc) < k) { tau = floor; first = -1; }
+    }
+    for (int bit = first; bit >= 0; --bit) {
       const uint32_t cand = tau | (1u << bit);
+      if (FLOOR && cand <= floor) { tau = cand; continue; }
       int cnt = 0;
       for (int i = threadIdx.x; i < v; i += ST) cnt += ordered_key(x[i]) >= cand;
       if (block_sum_i(cnt, sc) >= k) tau = cand;
@@ -312,7 +322,7 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int v,
     if (threadIdx.x == 0) out[b] = r;
     return;
   }
-  sample_in_memory(row, work + (size_t)b * v, v, temp, top_k[b], top_p[b], uniform_from(seeds[b], counters[b]), out + b, sc);
+  sample_in_memory<false>(row, work + (size_t)b * v, v, temp, top_k[b], top_p[b], uniform_from(seeds[b], counters[b]), 0, out + b, sc);
 }
 
 // ---------------------------------------------------------------- rows of at most 32,768 logits: the row in registers
@@ -328,11 +338,14 @@ sample_kernel(const float* __restrict__ logits, float* __restrict__ work, int v,
 //   draw    The chunks that hold a weight are scanned at once: in every warp, over the warps' sums of a chunk by one
 //           warp per chunk, and over the chunks' sums by every thread that holds a weight.
 // Without a top-k every id has a weight: those rows search the cut over bit patterns, in registers.
-// Lists that do not fit (ties, k > 200 or so) take the passes over memory.
+// k above 256 takes the passes over memory, before the row is read; so do lists that do not fit (many equal values, large
+// values side by side in few threads), with what the bound tells.
 // Every floating-point sum has the operands and the tree of sample_in_memory (terms left out are zeros there), so the
 // same id is chosen.  us per call, this kernel / the passes over memory: 64 rows
-// of 32,000, k 50, p 0.95 20 / 198; k 200, p 0.9 34 / 200; no top-k, p 0.9 44 / 102; one row 19 / 135; 64 of 8,000 15 / 76.
-constexpr int LISTED = 256;   // values that are ranked against one another
+// of 32,000, k 50, p 0.95 20 / 139; k 200, p 0.9 34 / 140; k 256 41 / 140; logits rounded to whole numbers, k 200 111 / 146;
+// no top-k, p 0.9 44 / 71; one row 19 / 135; 64 of 8,000 15 / 58.
+constexpr int MOST_K = 256;    // the largest k whose values are ranked against one another
+constexpr int LISTED = 352;   // ... and how many may be listed: 294 +- 6 reach the bound at k = 256 where they lie at random
 constexpr int OWN = 4;        // ... and of them per thread
 
 struct RowScratch {
@@ -376,26 +389,11 @@ __device__ __forceinline__ void scan_chunks(RowScratch& sc, int chunks) {
   __syncthreads();
 }
 
+// False (for the whole block) where the list does not fit; `floor` then is a key that at least k values reach.
 template <int NV>   // values per thread
-__global__ void __launch_bounds__(ST)
-sample_row_kernel(const float* __restrict__ logits, float* __restrict__ work, int v, const float* __restrict__ temperature,
-                  const int* __restrict__ top_k, const float* __restrict__ top_p,
-                  const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ counters,
-                  int* __restrict__ out, const int* __restrict__ status) {
-  __shared__ RowScratch sc;
-  pdl_trigger();
-  pdl_wait();
-  forward_status(status, out);
-  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const float* row = logits + (size_t)b * v;
-  const float temp = temperature[b];
-  if (!(temp > 0.f)) {
-    const int r = block_argmax(row, v, sc.block);
-    if (tid == 0) out[b] = r;
-    return;
-  }
-  const int k = top_k[b];
-  const float p = top_p[b], u = uniform_from(seeds[b], counters[b]);
+__device__ __forceinline__ bool sample_in_registers(const float* __restrict__ row, int v, float temp, int k, float p, float u,
+                                                    uint32_t& floor, int* __restrict__ out, RowScratch& sc) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t one = __float_as_uint(1.0f);
   int turn = 0;
   if (tid == 0) { sc.listed = 0; sc.overflow = 0; sc.choice = 0x7fffffff; sc.last = -1; }
@@ -416,11 +414,10 @@ sample_row_kernel(const float* __restrict__ logits, float* __restrict__ work, in
 
   if (k > 0 && k < v) {
     uint32_t bound = 0;
-    if (k <= LISTED)
-      for (int bit = 31; bit >= 0; --bit) {
-        const uint32_t cand = bound | (1u << bit);
-        if (__syncthreads_count(best >= cand) >= k) bound = cand;
-      }
+    for (int bit = 31; bit >= 0; --bit) {
+      const uint32_t cand = bound | (1u << bit);
+      if (__syncthreads_count(best >= cand) >= k) bound = cand;
+    }
     uint32_t mine = 0;      // chunks in which this thread's value reaches the bound
     if (bound != 0 && best >= bound) {
 #pragma unroll
@@ -437,8 +434,8 @@ sample_row_kernel(const float* __restrict__ logits, float* __restrict__ work, in
     __syncthreads();
     const int total = sc.listed;
     if (bound == 0 || sc.overflow != 0 || total > LISTED) {    // (uniform)
-      sample_in_memory(row, work + (size_t)b * v, v, temp, k, p, u, out + b, sc.block);
-      return;
+      floor = bound;
+      return false;
     }
 #pragma unroll
     for (int j = 0; j < OWN; ++j) {
@@ -535,8 +532,8 @@ sample_row_kernel(const float* __restrict__ logits, float* __restrict__ work, in
       if (last >= 0) atomicMax(&sc.last, last);
     }
     __syncthreads();
-    if (tid == 0) out[b] = sc.choice != 0x7fffffff ? sc.choice : sc.last;
-    return;
+    if (tid == 0) *out = sc.choice != 0x7fffffff ? sc.choice : sc.last;
+    return true;
   }
 
   // every id has a weight
@@ -587,7 +584,35 @@ sample_row_kernel(const float* __restrict__ logits, float* __restrict__ work, in
     atomicMax(&sc.last, (31 - __clz(weighted)) * ST + tid);
   }
   __syncthreads();
-  if (tid == 0) out[b] = sc.choice != 0x7fffffff ? sc.choice : sc.last;
+  if (tid == 0) *out = sc.choice != 0x7fffffff ? sc.choice : sc.last;
+  return true;
+}
+
+template <int NV>
+__global__ void __launch_bounds__(ST)
+sample_row_kernel(const float* __restrict__ logits, float* __restrict__ work, int v, const float* __restrict__ temperature,
+                  const int* __restrict__ top_k, const float* __restrict__ top_p,
+                  const unsigned long long* __restrict__ seeds, const unsigned long long* __restrict__ counters,
+                  int* __restrict__ out, const int* __restrict__ status) {
+  __shared__ RowScratch sc;
+  pdl_trigger();
+  pdl_wait();
+  forward_status(status, out);
+  const int b = blockIdx.x;
+  const float* row = logits + (size_t)b * v;
+  const float temp = temperature[b];
+  if (!(temp > 0.f)) {
+    const int r = block_argmax(row, v, sc.block);
+    if (threadIdx.x == 0) out[b] = r;
+    return;
+  }
+  const int k = top_k[b];
+  const float p = top_p[b], u = uniform_from(seeds[b], counters[b]);
+  uint32_t floor = 0;
+  if (k > MOST_K && k < v)    // more values than are ranked: told before the row is read, which the passes do anyway
+    sample_in_memory<false>(row, work + (size_t)b * v, v, temp, k, p, u, 0, out + b, sc.block);
+  else if (!sample_in_registers<NV>(row, v, temp, k, p, u, floor, out + b, sc))
+    sample_in_memory<true>(row, work + (size_t)b * v, v, temp, k, p, u, floor, out + b, sc.block);
 }
 
 // The kernel by the length of the rows: registers hold 32 values per thread; longer rows take the passes over `work`.
