@@ -92,3 +92,44 @@ def test_a_producer_that_gives_up_waits_for_its_copies(name):
     """Every kernel that arms a barrier with the bytes of a copy ends its producer with the wait for the copies in flight."""
     kernels = [k for k in sources()[name].split("__global__")[1:] if "mbar_expect_tx(" in k]
     assert kernels and all("mbar_drain(" in k for k in kernels)
+
+
+ROUTE = r"""
+#include "attention_route.h"
+#include <cstdio>
+// tokens, longest, requests, keys, nq, nk, values -> rows per CTA
+int main() {
+  long long t, q, r, k;
+  int nq, nk, d;
+  while (std::scanf("%lld %lld %lld %lld %d %d %d", &t, &q, &r, &k, &nq, &nk, &d) == 7)
+    std::printf("%d ", tllm::attention_rows_per_cta(t, q, r, k, nq, nk, d > 64, 148));
+  return 0;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_rows_share_a_cta_only_where_that_was_measured_to_be_no_slower(tmp_path):
+    src, exe = tmp_path / "route.cpp", tmp_path / "route"
+    src.write_text(ROUTE)
+    res = subprocess.run(["g++", "-std=c++17", "-I", build.CSRC, "-o", str(exe), str(src)], capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr
+    cases = [
+        # decoded tokens of groups of four and more, prompts, portions behind a context
+        ((8, 1, 8, 700, 32, 4, 64), 4), ((8, 1, 0, 0, 32, 4, 64), 4), ((1, 1, 1, 300, 16, 4, 64), 4),
+        ((509, 509, 1, 509, 32, 4, 64), 16), ((60, 60, 1, 60, 32, 32, 128), 4), ((7, 7, 1, 1507, 32, 32, 128), 4),
+        ((4, 4, 1, 1504, 28, 4, 128), 4), ((64, 1, 64, 255, 32, 4, 64), 4), ((33, 33, 1, 33, 20, 4, 64), 4),
+        # a head with keys of its own, decoded: nothing is shared
+        ((8, 1, 8, 2000, 32, 32, 128), 0), ((3, 3, 1, 900, 16, 16, 64), 0),
+        # few keys
+        ((8, 1, 8, 9, 32, 4, 64), 0), ((4, 4, 1, 4, 32, 4, 64), 0), ((17, 17, 1, 17, 32, 32, 128), 0), ((64, 1, 64, 31, 32, 4, 64), 0),
+        # few requests whose tokens would be walked one after the other, and many of them
+        ((4, 1, 4, 700, 28, 4, 128), 0), ((24, 20, 5, 700, 32, 32, 128), 0), ((20, 4, 17, 1400, 32, 32, 128), 0),
+        ((24, 20, 5, 700, 12, 4, 64), 0), ((24, 20, 0, 700, 12, 4, 64), 0), ((16, 1, 16, 40, 28, 4, 128), 0),
+        ((16, 1, 16, 700, 28, 4, 128), 4), ((67, 4, 64, 1400, 8, 4, 64), 4), ((67, 4, 64, 1400, 32, 32, 128), 4),
+        # portions of several requests: each brings more rows than a CTA takes
+        ((72, 24, 3, 24, 12, 4, 64), 4), ((30, 10, 3, 900, 32, 32, 128), 4),
+    ]
+    text = "\n".join(" ".join(map(str, c)) for c, _ in cases)
+    got = subprocess.run([str(exe)], input=text, capture_output=True, text=True, timeout=60).stdout.split()
+    assert [int(g) for g in got] == [want for _, want in cases]

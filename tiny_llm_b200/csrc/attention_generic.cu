@@ -28,6 +28,7 @@
 // absolute key index (:63-66, :402-405).
 #include <math_constants.h>
 
+#include "attention_route.h"
 #include "common.cuh"
 
 TLLM_DEFINE_LAST_ERROR
@@ -788,14 +789,16 @@ using namespace tllm;
 // visible inside the query's chunk of positions only.  out_f32 != 0: the output rows are float32 whatever the cache's type.
 // `sink` (float32, one per query head, or null): exp(sink) joins every softmax's denominator of that head.
 // `keep`: the first positions that a window leaves visible; `rel` (float32 [nq, rel_len] or null): a bias per head and
-// distance.  `max_q_len`: the most tokens of one request in the step (how many rows share their keys; 0 if unknown).
+// distance.  `max_q_len`: the most tokens of one request in the step (how many rows share their keys; 0 if unknown);
+// `max_kv_len`: the most keys of one request, or more, `n_requests` (0 if unknown): they choose the launch, see attention_route.h.
 extern "C" int tllm_paged_attention_maps(const void* q, int q_row_stride, const void* kcache, const void* vcache,
                                          const int* block_table, int max_blocks, const int* token_request,
                                          const int* positions, void* out, int n_tokens, int nq, int nkv, int maps, int kd,
                                          int vd, int page_size, long long k_page_stride, long long k_head_stride,
                                          long long v_page_stride, long long v_head_stride, float scale, int window,
                                          int chunk, int dtype, int out_f32, int split_override, const float* sink,
-                                         int keep, const float* rel, int rel_len, int max_q_len, void* stream) {
+                                         int keep, const float* rel, int rel_len, int max_q_len, int max_kv_len,
+                                         int n_requests, void* stream) {
   TLLM_REQUIRE(n_tokens > 0 && nq > 0 && nkv > 0 && nq % nkv == 0 && maps > 0,
                "attention: %d tokens, %d heads, %d key/value heads (heads must be a multiple of key/value heads)", n_tokens, nq, nkv);
   TLLM_REQUIRE(kd >= 1 && kd <= MAX_KD && vd >= 1 && vd <= MAX_VD,
@@ -815,14 +818,17 @@ extern "C" int tllm_paged_attention_maps(const void* q, int q_row_stride, const 
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     TLLM_FAIL(TLLM_ERR_CUDA, "attention: cannot read the number of SMs");
-  // Rows that share their keys: a CTA takes 16 of them where that gives every SM one, else 4 (decoded tokens: with 16, half
-  // of the SMs would idle and the chain of one CTA would be longer); fewer than 4 that share keep the launches below.
-  const long long shared_rows = (long long)max_q_len * (nq / nkv), all_rows = (long long)n_tokens * (nq / nkv);
+  // Rows that share their keys: several to a CTA
+  const long long all_rows = (long long)n_tokens * (nq / nkv);
+  long long keys = max_kv_len;
+  if (keys > 0 && window > 0 && keys > (long long)window + g.keep) keys = (long long)window + g.keep;
+  if (keys > 0 && chunk > 0 && keys > chunk) keys = chunk;
+  const int rows = split_override < 0 ? attention_rows_per_cta(n_tokens, max_q_len, n_requests, keys, g.nq, g.nk, kd > 64 || vd > 64, sms)
+                                      : (split_override == 3 ? 16 : (split_override == 4 ? 4 : 0));
   const bool vvec = vd % 4 == 0 && ((size_t)vcache % 16) == 0 && v_page_stride % 4 == 0 && v_head_stride % 4 == 0;
-  if (dtype == TLLM_F32 && g.kvec && vvec && kd <= 128 && vd <= 128 &&
-      (split_override < 0 ? shared_rows >= 4 : split_override == 3 || split_override == 4)) {
+  if (dtype == TLLM_F32 && g.kvec && vvec && kd <= 128 && vd <= 128 && rows > 0) {
     const long long wide = (all_rows + 15) / 16 * g.nk, narrow = (all_rows + 3) / 4 * g.nk;
-    const bool r16 = split_override < 0 ? shared_rows >= 16 && wide >= sms : split_override == 3;
+    const bool r16 = rows == 16;
     TLLM_REQUIRE(narrow <= 2147483647LL, "attention: %lld (token, head) pairs exceed the grid", tasks);
     cudaStream_t s = (cudaStream_t)stream;
 #define TLLM_ATT_ROWS(OD_, R_)                                                                                         \
@@ -860,7 +866,8 @@ extern "C" int tllm_paged_attention_generic(const void* q, int q_row_stride, con
                                             const int* block_table, int max_blocks, const int* token_request,
                                             const int* positions, void* out, int n_tokens, int nq, int nkv, int hd,
                                             int page_size, long long page_stride, long long head_stride,
-                                            float scale, int window, int dtype, int split_override, int max_q_len, void* stream) {
+                                            float scale, int window, int dtype, int split_override, int max_q_len,
+                                            int max_kv_len, int n_requests, void* stream) {
   TLLM_REQUIRE(hd >= 16 && hd <= MAX_HD && hd % 16 == 0,
                "attention: head size %d is not built (multiples of 16 up to %d are)", hd, MAX_HD);
   const int elem = dtype == TLLM_F32 ? 4 : 2;
@@ -868,5 +875,6 @@ extern "C" int tllm_paged_attention_generic(const void* q, int q_row_stride, con
                "attention: cache rows must be 16-byte aligned");
   return tllm_paged_attention_maps(q, q_row_stride, kcache, vcache, block_table, max_blocks, token_request, positions, out,
                                    n_tokens, nq, nkv, 1, hd, hd, page_size, page_stride, head_stride, page_stride, head_stride,
-                                   scale, window, 0, dtype, 0, split_override, nullptr, 0, nullptr, 0, max_q_len, stream);
+                                   scale, window, 0, dtype, 0, split_override, nullptr, 0, nullptr, 0, max_q_len, max_kv_len, n_requests,
+                                   stream);
 }

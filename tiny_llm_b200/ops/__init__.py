@@ -1593,7 +1593,8 @@ def paged_attention(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, head_d
         _ptr(batch.token_request), _ptr(batch.positions), _ptr(out), t, num_heads, num_kv_heads, head_dim,
         page_size, ctypes.c_longlong(k_cache.stride(0)), ctypes.c_longlong(k_cache.stride(1)),
         ctypes.c_float(scale), int(window or 0), _code(qkv.dtype),
-        -1 if generic_attention_split is None else int(generic_attention_split), int(getattr(batch, "max_q_len", 0)), _stream())
+        -1 if generic_attention_split is None else int(generic_attention_split), int(getattr(batch, "max_q_len", 0)),
+        int(getattr(batch, "max_kv_len", 0)), int(getattr(batch, "num_requests", 0)), _stream())
 
 
 # bfloat16 attention with several score maps per head on the tensor cores (False: the CUDA-core kernel; for measurements)
@@ -1678,7 +1679,8 @@ def paged_attention_maps(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, m
           ctypes.c_longlong(v_cache.stride(0)), ctypes.c_longlong(v_cache.stride(1)), ctypes.c_float(scale),
           int(window or 0), int(chunk or 0), _code(qkv.dtype), 1 if out.dtype == torch.float32 else 0,
           -1 if generic_attention_split is None else int(generic_attention_split), _ptr(sink), keep_first, _ptr(rel), rel_len,
-          int(getattr(batch, "max_q_len", 0)), _stream())
+          int(getattr(batch, "max_q_len", 0)), int(getattr(batch, "max_kv_len", 0)),
+          int(getattr(batch, "num_requests", 0)), _stream())
 
 
 def attention_tc_timing(head_dim: int = 64) -> Optional[dict]:
