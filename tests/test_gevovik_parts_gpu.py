@@ -348,6 +348,69 @@ def test_streamed_recurrence_gives_the_bits_of_the_general_kernel(mode, sizes):
     ops.check_status()
 
 
+@pytest.mark.parametrize("mode,sizes,lens", [
+    ("delta", (3, 3, 64, 33), [1] * 6), ("delta", (3, 3, 64, 33), [1, 2, 1]), ("delta", (2, 1, 60, 20), [1] * 4),
+    ("delta", (4, 1, 68, 48), [0, 1, 7, 8, 9, 77]), ("delta", (4, 2, 132, 17), [33, 1, 40]),
+    ("channel_decay", (3, 3, 64, 33), [0, 1, 7, 8, 9, 77]), ("channel_decay", (3, 3, 60, 16), [9, 1]),
+    ("channel_decay", (2, 2, 68, 20), [1] * 5), ("channel_decay", (2, 1, 256, 20), [31, 50]),
+    ("state_space", (2, 1, 4, 5), [64, 31, 1]), ("state_space", (4, 2, 36, 16), [32, 32]), ("state_space", (4, 2, 36, 16), [32, 31]),
+    ("state_space", (3, 3, 64, 33), [1] * 6), ("state_space", (2, 2, 128, 20), [0, 1, 7, 8, 9, 77])])
+def test_recurrence_gives_the_same_bits_on_both_sides_of_the_lines_between_its_kernels(mode, sizes, lens):
+    """Key sizes around 64, decoded tokens alone, portions of about 32 tokens: what chooses between the streamed and the
+    general kernel.  Rows that start off a 16-byte boundary always take the general one."""
+    from tiny_llm_b200 import ops
+    heads, kvh, kd, vd = sizes
+    g, n = torch.Generator().manual_seed(kd + len(lens)), sum(lens)
+    q, k, v = (x.reshape(n, -1).contiguous() for x in recurrence_inputs(g, n, heads, kvh, kd, vd))
+    gb = torch.rand(n, heads, 2, generator=g) * 0.9 + 0.05
+    gk = torch.rand(n, heads * kd, generator=g).to(DEV) if mode == "channel_decay" else None
+    if gk is not None:
+        gb[..., 0] = 1.0
+    states, b = torch.randn(len(lens), heads, vd, kd, generator=g), batch_of(lens, [0] * len(lens))
+    got = []
+    for first in (0, 1):
+        place = torch.empty(q.numel() + first, device=DEV)
+        place[first:] = q.to(DEV).reshape(-1)
+        state, out = states.to(DEV), torch.zeros(n, heads * vd, device=DEV)
+        ops.delta_rule_scan(place[first:].view(q.shape), k.to(DEV), v.to(DEV), gb.to(DEV), state, b, heads, kvh, kd, vd, out,
+                            mode=mode, gk=gk)
+        got.append((out, state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("mode", ["delta", "state_space", "channel_decay"])
+@pytest.mark.parametrize("off_boundary", ["state", "gb"])
+@pytest.mark.parametrize("sizes", [(3, 3, 64, 33), (4, 1, 128, 48), (2, 2, 252, 20)])
+def test_general_recurrence_with_rows_on_16_bytes_gives_the_same_bits(mode, off_boundary, sizes):
+    """Keys on 16 bytes beside states that start four bytes past such a boundary, or decays and step sizes that start four
+    bytes past an 8-byte one: the general kernel, which then copies whole pieces of the keys' rows."""
+    from tiny_llm_b200 import ops
+    heads, kvh, kd, vd = sizes
+    lens = [0, 1, 7, 8, 9, 77]
+    g, n = torch.Generator().manual_seed(kd + len(mode)), sum(lens)
+    q, k, v = (x.reshape(n, -1).contiguous() for x in recurrence_inputs(g, n, heads, kvh, kd, vd))
+    gb = torch.rand(n, heads, 2, generator=g) * 0.9 + 0.05
+    gk = torch.rand(n, heads * kd, generator=g).to(DEV) if mode == "channel_decay" else None
+    if gk is not None:
+        gb[..., 0] = 1.0
+    states = torch.randn(len(lens), heads, vd, kd, generator=g)
+    b = batch_of(lens, [0] * len(lens))
+
+    def place(name, x):
+        y = torch.empty(x.numel() + 1, device=DEV)
+        first = 1 if name == off_boundary else 0
+        y[first: first + x.numel()] = x.to(DEV).reshape(-1)
+        return y[first: first + x.numel()].view(x.shape)
+    got = []
+    for names in (("state", "gb"), (None, None)):
+        state, out = place(names[0], states), torch.zeros(n, heads * vd, device=DEV)
+        ops.delta_rule_scan(q.to(DEV), k.to(DEV), v.to(DEV), place(names[1], gb), state, b, heads, kvh, kd, vd, out, mode=mode, gk=gk)
+        got.append((out, state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    ops.check_status()
+
+
 @pytest.mark.parametrize("sizes", [(4, 2, 16, 16), (6, 3, 10, 6), (5, 5, 12, 8), (2, 1, 7, 20), (8, 2, 64, 32), (16, 16, 32, 8)])
 def test_state_space_recurrence_and_the_gated_norm_in_parts(sizes):
     from tiny_llm_b200 import ops

@@ -649,7 +649,7 @@ extern "C" int tllm_conv_state_update(const void* proj, int ld, float* kept, con
 
 extern "C" int tllm_delta_rule_scan(const float* q, const float* k, const float* v, const float* gb, float* state,
                                     const int* slots, const int* cu_q, float* out, int heads, int kv_heads, int kd, int vd,
-                                    int n_requests, int mode, const float* gk, int* status, void* stream) {
+                                    int n_requests, int n_tokens, int mode, const float* gk, int* status, void* stream) {
   TLLM_REQUIRE(n_requests > 0 && n_requests <= 65535 && heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0,
                "delta_rule_scan: %d requests, %d heads over %d query/key heads", n_requests, heads, kv_heads);
   TLLM_REQUIRE(kd >= 1 && kd <= 256 && vd >= 1, "delta_rule_scan: key size %d (at most 256), value size %d", kd, vd);
@@ -659,15 +659,25 @@ extern "C" int tllm_delta_rule_scan(const float* q, const float* k, const float*
   TLLM_REQUIRE(mode >= 0 && mode <= 2 && (mode == 2) == (gk != nullptr), "delta_rule_scan: mode %d (0, 1 or 2; decays per key channel with 2 only)", mode);
   const dim3 grid((vd + DR_COLS - 1) / DR_COLS, heads, n_requests);
   cudaStream_t s = (cudaStream_t)stream;
-  // key rows, decays and state columns of whole 16-byte pieces: the streamed kernel
-  if ((kd & 3) == 0 && status != nullptr && (((size_t)q | (size_t)k | (size_t)gk | (size_t)state) & 15) == 0 && ((size_t)gb & 7) == 0) {
+  // The streamed kernel: key rows, decays and state columns of whole 16-byte pieces, and sizes where it is the faster one.
+  // With key rows of less than 64 its fifth warp and its ring cost more than they save (us, streamed / general, values of 64,
+  // keys of 36: 64 requests of one token, 32 heads, 38 / 22, of eight 56 / 43; 500 tokens 82 / 71; 32: 19 / 18, 39 / 37,
+  // 76 / 67), except for the state-space form over portions, whose chain it shortens most (16: 500 tokens 47 / 55, 61 tokens
+  // 7.4 / 8.7; eight requests of 16 12 / 10).  64: the streamed one (mode 1, 500 tokens 46 / 55; mode 2, 61 tokens 11.5 /
+  // 12.8; decoded tokens 18 / 19), but for tokens of the delta rule where CTAs share SMs: 500 tokens 69 / 72 with 16 heads,
+  // 82 / 72 with 32; eight requests of eight 4.3 / 4.9 with 8 heads, 6.4 / 5.9 with 16.  Above 64 it takes 0.2 to 0.9 of the
+  // time (68 or 132 with 64 requests of one token and 32 heads 1.08).
+  const bool decodes = n_tokens <= n_requests, portions = n_tokens >= 32LL * n_requests;
+  const long long ctas = (long long)grid.x * heads * n_requests;
+  const bool streamed = kd > 64 || (kd == 64 && (mode != 0 || decodes || ctas <= (portions ? 74 : 296))) || (mode == 1 && portions);
+  if (streamed && (kd & 3) == 0 && status != nullptr && (((size_t)q | (size_t)k | (size_t)gk | (size_t)state) & 15) == 0 && ((size_t)gb & 7) == 0) {
 #define TLLM_STREAM(R)                                                            \
   do {                                                                            \
     if (mode == 0) return launch_stream<R, 0>(a, grid, status, s);                \
     if (mode == 1) return launch_stream<R, 1>(a, grid, status, s);                \
     return launch_stream<R, 2>(a, grid, status, s);                               \
   } while (0)
-    if (kd <= 32) TLLM_STREAM(4);
+    if (kd <= 32) return launch_stream<4, 1>(a, grid, status, s);   // (see above: mode 1 alone)
     if (kd <= 64) TLLM_STREAM(8);
     if (kd <= 128) TLLM_STREAM(16);
     TLLM_STREAM(32);

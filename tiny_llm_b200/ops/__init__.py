@@ -961,7 +961,7 @@ def delta_rule_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gb: torch
         raise KernelError("delta_rule_scan: shapes or dtypes do not fit")
     lib = build.load_library("delta_rule")
     _call(lib, lib.tllm_delta_rule_scan, _ptr(q), _ptr(k), _ptr(v), _ptr(gb), _ptr(state), _ptr(batch.slots),
-          _ptr(batch.cu_q), _ptr(out), heads, kv_heads, key_dim, value_dim, batch.num_requests, PREPARE_MODES[mode],
+          _ptr(batch.cu_q), _ptr(out), heads, kv_heads, key_dim, value_dim, batch.num_requests, t, PREPARE_MODES[mode],
           _ptr(gk), _ptr(status_word(q.device)), _stream())
 
 
