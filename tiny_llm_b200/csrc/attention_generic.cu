@@ -343,7 +343,9 @@ paged_attention_grouped_kernel(const T* __restrict__ q, int q_row_stride, const 
 // through fma.rn.f32x2, whose halves round like fmaf.  The sums over a tile's 32 keys keep the tree of warp_sum: partners
 // exchange halves of the rows instead of whole rows, so 16 rows take 16 steps of shuffles instead of 80 and 4 rows 6
 // instead of 20.  us per layer at the TinyLlama sizes, this kernel / the launches above: a prompt of 509 tokens 110 / 351,
-// eight decoded tokens at context 700 18 / 42.
+// eight decoded tokens at context 700 18 / 42.  What bounds it: the latencies of the eight warps that an SM has (the tiles
+// take 144 to 164 KB, so one CTA); at 509 tokens issue slots are 27 % used, the load/store pipe 20 %, shared memory 34 %,
+// and a quarter of a warp's time is the merge, where ways with fewer tiles wait.
 __device__ __forceinline__ uint64_t pack_pair(float lo, float hi) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));

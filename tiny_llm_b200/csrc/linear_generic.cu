@@ -294,8 +294,9 @@ static int launch_tiled(const float* a, const float* w, float* out, int m, int n
 // lie 128 bytes apart and 16-byte reads of eight rows do not collide), KB boxes per stage; a producer warp issues them,
 // the weights' first stages before the wait for earlier kernels.  A lane owns one weight row and TR rows of A: TR chains of
 // fmaf, whose operands it reads KS steps of four k ahead (read where they are used, every step stood behind a trip to
-// shared memory).  What bounds it: the weights from memory where there are many rows of them, else the reads of shared
-// memory (1 + TR per four k); the chains themselves (4 cycles per k) would take 4.3 us at K = 2,048.
+// shared memory).  What bounds it: the weights from memory where there are many rows of them, else the latencies of the few
+// warps that an SM has (8 x 2,048 x 5,632: 3.3 warps, issue slots 16 % used, the load/store pipe 12 %; 8 x 11,264 x 2,048:
+// 6.7, 26 and 19 %); the chains themselves (4 cycles per k) would take 4.3 us at K = 2,048.
 // us, this kernel / one chain per thread with cp.async by the computing threads (m = 8): 2,560 x 2,048 14.9 / 26.8,
 // 2,048 x 2,048 13.8 / 20.2, 11,264 x 2,048 27.4 / 43.5, 2,048 x 5,632 34.2 / 55.0, 32,000 x 2,048 74.6 / 115.7; m = 1:
 // 9.0 / 18.3, 8.5 / 17.4, 23.8 / 26.9, 19.9 / 43.2, 46.9 / 50.0.
@@ -459,9 +460,15 @@ int launch_skinny(const float* a, const float* w, float* out, int m, int n, int 
   return TLLM_OK;
 }
 
-// Which shape: few weight rows want small CTAs (more SMs at work), many want the weight rows' reads shared by more rows of A
-// (8 x 11,264 x 2,048: 16 weight rows per warp 27.4 us, 8 41.9; 8 x 2,048 x 2,048: 20 and 13.8; the line between at
-// 8,192 weight rows is where both leave no SM idle).
+// Which shape: few weight rows want small CTAs (more SMs at work), many want the weight rows' reads shared by more rows of A.
+// A wave of the small CTAs is 4,736 weight rows at m = 5 to 8 (four per SM), of the large ones 14,208, and a large one takes
+// about twice as long.  K = 2,048, us, small / large, weights not in the L2:
+//   weight rows   2,048        4,096        5,120        8,192        10,240       16,384       32,000
+//   m = 1         7.6 / 10.6   9.1 / 11.2   16 / 12      18 / 13      26 / 24      35 / 26      65 / 51
+//   m = 8         13 / 21      14 / 24      25 / 26      29 / 27      41 / 28      56 / 54      99 / 83
+//   m = 16        19 / 33      20 / 40      38 / 42      40 / 44      59 / 45      80 / 88      140 / 133
+// So the line may lie anywhere from 4,736 to 9,472 for eight rows; one row would take the large shape from 4,736 on, and 16
+// rows the small one up to 9,472.  (K = 5,632 gives the same picture.)  Two to four rows were measured in one shape only.
 static int launch_skinny_rows(const float* a, const float* w, float* out, int m, int n, int k, int lda, int ldo, int mode, int* status, cudaStream_t s) {
   const bool many = n >= 8192;
   if (m <= 1) return many ? launch_skinny<1, 32, 1, 1, 2, 8>(a, w, out, m, n, k, lda, ldo, mode, status, s)
