@@ -97,7 +97,7 @@ def replay_tape(tape) -> None:
 def knobs():
     """The module's switches that decide which kernels a step launches; a tape or graph holds for one setting of them."""
     return (force_generic, split_k, cluster_mask, attention_tc, decode_wide_ctas, decode_cluster_merge, qkv_fused_rows,
-            linear_skinny, generic_attention_split, split_mixed_attention, min_gru_segment, linear_attention_segment, moe_mma, moe_wide_tiles, moe_tc_rows_per_expert, window_attention_tc, window_attention_splits, attention_maps_tc, attention_maps_decode_pairs, attention_maps_splits, attention_talk_tc, attention_talk_splits, attention_talk_stages, _pdl)
+            linear_skinny, attention_decode_tma, generic_attention_split, split_mixed_attention, min_gru_segment, linear_attention_segment, moe_mma, moe_wide_tiles, moe_tc_rows_per_expert, window_attention_tc, window_attention_splits, attention_maps_tc, attention_maps_decode_pairs, attention_maps_splits, attention_talk_tc, attention_talk_splits, attention_talk_stages, _pdl)
 
 
 def _i32(t: Optional[torch.Tensor], name: str):
@@ -1230,7 +1230,8 @@ _STATUS_CODES = {1: "TMA producer of a tensor-core product", 2: "MMA issuer of a
                  7: "TMA producer of the tensor-core attention", 8: "MMA issuer of the tensor-core attention",
                  9: "softmax of the tensor-core attention",
                  10: "TMA producer of a streamed 32-bit product", 11: "computing warp of a streamed 32-bit product",
-                 12: "copying warp of a delta-rule or state-space scan", 13: "computing warp of a delta-rule or state-space scan"}
+                 12: "copying warp of a delta-rule or state-space scan", 13: "computing warp of a delta-rule or state-space scan",
+                 18: "TMA producer of the attention of decoded tokens", 19: "computing warp of the attention of decoded tokens"}
 
 
 def raise_status(device, code: int) -> None:
@@ -1503,6 +1504,29 @@ def _wide_splits(num_requests: int, num_kv_heads: int, max_kv_len: int) -> int:
     return splits if ctas < lo and hi > 0 and _cluster_merge(num_requests, num_kv_heads, splits) else 0
 
 
+# Decoded tokens of head size 64 or 128 without a window, pages of at most a tile: the kernel that fetches its tiles by TMA
+# (csrc/attention_decode.cu), in slices of at most eight tiles by smaller CTAs, three to an SM, else by larger ones, two to an
+# SM; as many slices (up to the 8 of a portable cluster) as one wave of CTAs holds, one tile per warp at least.  us per launch,
+# this kernel / the ones above: 4 key rows of 64, 64 requests with 300, 700, 1,400 keys 6.9 / 11.7, 9.9 / 17.4, 15.9 / 23.7,
+# 16 with 1,400 7.7 / 11.6, 8 with 1,400 6.4 / 6.5, 1 with 300 4.6 / 5.2; 8 key rows of 128, 16 requests with 1,400 and
+# 5,600 18.6 / 25.4, 56.0 / 71.7.  Not where eight slices leave SMs idle and are long, which the merge by a kernel of its own
+# can cut finer: 8 x 128, 5,600 keys, one request 15.9 / 12.6, two 17.3 / 15.3, four (256 CTAs) 19.0 / 27.5.
+# TLLM_ATTENTION_DECODE_TMA=0 turns it off (a switch for measurements).
+attention_decode_tma = os.environ.get("TLLM_ATTENTION_DECODE_TMA", "1") != "0"
+
+
+def _decode_slices(num_requests: int, num_kv_heads: int, head_dim: int, max_kv_len: int):
+    """(slices of keys, whether they are a few tiles each) for the TMA kernel, or None where it is not taken."""
+    tiles = max(1, -(-max_kv_len * head_dim // 4096))        # of 64 keys of 64 values, or 32 of 128
+    items, sms = num_requests * num_kv_heads, sm_count()
+    for few, ctas, warps in ((True, 3 * sms, 4), (False, 2 * sms, 6)):
+        s = max(1, min(8, ctas // items, -(-tiles // warps)))
+        per = -(-tiles // s)
+        if not few or per <= 8:
+            s = -(-tiles // per)
+            return None if per > 12 and items * s < sms else (s, few)
+
+
 # The attention of the 32-bit path runs 16 or 4 rows that share their keys per CTA, eight warps per (token, head), or one
 # warp per (token, key/value head, four query heads), by sizes and numbers; all give the same bits.  3 / 4 force the first
 # two (key and value rows of up to 128 values), True / False the others, 2 the plainest form (one warp per pair); tests
@@ -1565,6 +1589,18 @@ def paged_attention(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, head_d
                 _ptr(block_table), block_table.shape[1], _ptr(batch.cu_q), _ptr(batch.q_start), _ptr(out), t,
                 batch.num_requests, batch.max_q_len, num_heads, num_kv_heads, head_dim, page_size,
                 ctypes.c_float(scale), _ptr(status_word(qkv.device)), _stream())
+            return
+    if qkv.dtype == torch.bfloat16 and not force_generic and attention_decode_tma and head_dim in ATTENTION_TC_HEAD_DIMS and \
+            not window and batch.max_q_len * group <= 16 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and \
+            k_cache.is_contiguous() and v_cache.is_contiguous():
+        lib = build.load_library("attention_decode", flags=(f"-DTLLM_HEAD_DIM={head_dim}",))
+        slices = _decode_slices(batch.num_requests, num_kv_heads, head_dim, batch.max_kv_len)
+        if slices and lib.tllm_attention_decode_fits(num_heads, num_kv_heads, head_dim, page_size, batch.max_q_len):
+            _call(lib, lib.tllm_attention_decode,
+                _ptr(qkv), qkv.stride(0), _ptr(k_cache), _ptr(v_cache), ctypes.c_longlong(k_cache.shape[0]),
+                _ptr(block_table), block_table.shape[1], _ptr(batch.cu_q), _ptr(batch.q_start), _ptr(out),
+                batch.num_requests, batch.max_q_len, num_heads, num_kv_heads, head_dim, page_size, ctypes.c_float(scale),
+                slices[0], int(slices[1]), _ptr(status_word(qkv.device)), _stream())
             return
     if qkv.dtype == torch.bfloat16 and not force_generic and head_dim % 16 == 0 and 16 <= head_dim <= 256 and \
             qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0:
@@ -1758,6 +1794,8 @@ def build_all(verbose: bool = True):
     paths += [build.compile_library("attention_mma", flags=(f"-DTLLM_HEAD_DIM={hd}",), verbose=verbose)
               for hd in ATTENTION_HEAD_DIMS]
     paths += [build.compile_library("attention_tc", flags=(f"-DTLLM_HEAD_DIM={hd}",), verbose=verbose)
+              for hd in ATTENTION_TC_HEAD_DIMS]
+    paths += [build.compile_library("attention_decode", flags=(f"-DTLLM_HEAD_DIM={hd}",), verbose=verbose)
               for hd in ATTENTION_TC_HEAD_DIMS]
     paths += [build.compile_library("attention_maps_mma", flags=(f"-DTLLM_HEAD_DIM={kd}", f"-DTLLM_VALUE_DIM={vd}"), verbose=verbose)
               for kd, vd in ATTENTION_MAPS_DIMS]
