@@ -395,7 +395,11 @@ __device__ __forceinline__ float reduce_rows(const float (&in)[R], Op op, int la
 
 template <int OD, int R>
 struct RowsSmem {
-  static constexpr bool TWO = OD <= 2;                       // keys and values of a tile in buffers of their own
+  // Keys and values of a tile in buffers of their own, or values over the keys that have been multiplied.  Sixteen rows of up
+  // to 64 values: with one buffer two CTAs share an SM (97 KB of shared memory, 128 registers), and one computes while the
+  // other waits; with two buffers one CTA had an SM for itself (32 heads over 4 of 64, us: 131 tokens 24.1 -> 16.6, 509
+  // 108.9 -> 76.1, 2,048 1,007 -> 698, 300 beside eight decoded ones 107.7 -> 90.9).
+  static constexpr bool TWO = OD <= 2 && R < 16;
   static constexpr int K_LD = OD * 32 + 4, V_LD = OD * 32, P_LD = R + 4;   // pitches that keep 16-byte accesses apart
   static constexpr int K_FLOATS = 32 * K_LD, V_FLOATS = TWO ? 32 * V_LD : 0, P_FLOATS = 32 * P_LD;
   static constexpr int WARP_FLOATS = K_FLOATS + V_FLOATS + P_FLOATS;
