@@ -1,5 +1,5 @@
 // C[M,N] = A[M,K] . W[N,K]^T on the CUDA cores with 32-bit accumulation (FFMA only, no tensor-core
-// mode): the product of the true 32-bit path, and the fallback of the bfloat16 path for sizes the
+// mode): the products of the 32-bit path that linear_f32_tc.cu does not take, and the fallback of the bfloat16 path for sizes the
 // tensor-core kernels refuse.  Any M, N, K.  Every output element is ONE chain of fmaf over k in
 // ascending order starting from zero, whatever M is and whichever of the kernels below computes it,
 // so a row's result does not depend on its batch, to the bit.

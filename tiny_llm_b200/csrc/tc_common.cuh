@@ -21,6 +21,7 @@ constexpr int ERR_PRODUCER = 1, ERR_MMA = 2, ERR_EPILOGUE = 3;                  
 constexpr int ERR_ATT_PRODUCER = 7, ERR_ATT_MMA = 8, ERR_ATT_SOFTMAX = 9;       // tensor-core attention (attention_tc.cu)
 constexpr int ERR_SK_PRODUCER = 10, ERR_SK_CONSUMER = 11;                       // streamed 32-bit products (linear_generic.cu)
 constexpr int ERR_DR_PRODUCER = 12, ERR_DR_CONSUMER = 13;                       // streamed scans (delta_rule.cu)
+constexpr int ERR_FT_PRODUCER = 14, ERR_FT_MMA = 15, ERR_FT_SPLIT = 16, ERR_FT_SUMS = 17;   // 32-bit products on the tensor cores (linear_f32_tc.cu)
 constexpr int ERR_AD_PRODUCER = 18, ERR_AD_CONSUMER = 19;                       // attention of decoded tokens (attention_decode.cu)
 
 // ---------------------------------------------------------------- PTX wrappers

@@ -97,7 +97,7 @@ def replay_tape(tape) -> None:
 def knobs():
     """The module's switches that decide which kernels a step launches; a tape or graph holds for one setting of them."""
     return (force_generic, split_k, cluster_mask, attention_tc, decode_wide_ctas, decode_cluster_merge, qkv_fused_rows,
-            linear_skinny, attention_decode_tma, generic_attention_split, split_mixed_attention, min_gru_segment, linear_attention_segment, moe_mma, moe_wide_tiles, moe_tc_rows_per_expert, window_attention_tc, window_attention_splits, attention_maps_tc, attention_maps_decode_pairs, attention_maps_splits, attention_talk_tc, attention_talk_splits, attention_talk_stages, _pdl)
+            linear_skinny, linear_f32_tc, attention_decode_tma, generic_attention_split, split_mixed_attention, min_gru_segment, linear_attention_segment, moe_mma, moe_wide_tiles, moe_tc_rows_per_expert, window_attention_tc, window_attention_splits, attention_maps_tc, attention_maps_decode_pairs, attention_maps_splits, attention_talk_tc, attention_talk_splits, attention_talk_stages, _pdl)
 
 
 def _i32(t: Optional[torch.Tensor], name: str):
@@ -1231,6 +1231,8 @@ _STATUS_CODES = {1: "TMA producer of a tensor-core product", 2: "MMA issuer of a
                  9: "softmax of the tensor-core attention",
                  10: "TMA producer of a streamed 32-bit product", 11: "computing warp of a streamed 32-bit product",
                  12: "copying warp of a delta-rule or state-space scan", 13: "computing warp of a delta-rule or state-space scan",
+                 14: "TMA producer of a 32-bit tensor-core product", 15: "MMA issuer of a 32-bit tensor-core product",
+                 16: "splitting warp of a 32-bit tensor-core product", 17: "summing warp of a 32-bit tensor-core product",
                  18: "TMA producer of the attention of decoded tokens", 19: "computing warp of the attention of decoded tokens"}
 
 
@@ -1337,9 +1339,24 @@ def fused_qkv_preferred(m: int, n: int, k: int) -> bool:
     return m <= qkv_fused_rows or m > 128 or _cluster_slices(n, k) < 8
 
 
-# float32 products whose rows start on 16 bytes take the streaming kernel (at most 16 rows) or tiles chosen by size;
-# False keeps the 64 x 64 tiles for all.  All give the same bits (tests compare them).
+# float32 products that stay off the tensor cores (below) and whose rows start on 16 bytes take the streaming kernel (at most
+# 16 rows) or tiles chosen by size; False keeps the 64 x 64 tiles for all of them.  All give the same bits (tests compare them).
 linear_skinny = True
+
+
+# float32 products of large weights on the tensor cores, every factor as three bfloat16 parts that add up to it exactly
+# (csrc/linear_f32_tc.cu): whole boxes, rows of at least 2,048 values, at least 2^20 weights.  The rule may not look at the
+# number of rows, since the kernels' sums have other bits.  us, one chain of fmaf / this: 512 x 2,048 one row 7.9 / 7.2, 16
+# 12.7 / 7.6, 100 38 / 15; 256 x 4,096 13.9 / 10.0, 23.5 / 10.4, 72 / 21; with shorter rows few rows of A lose more than many
+# gain: 1,024 x 1,024 4.8 / 7.3, 8.0 / 7.6, 20 / 14; 2,048 x 512 3.4 / 7.4, 6.2 / 7.5, 16 / 14.
+# TLLM_LINEAR_F32_TC=0 turns it off.
+linear_f32_tc = os.environ.get("TLLM_LINEAR_F32_TC", "1") != "0"
+
+
+def _f32_tc_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
+    n, k = w.shape
+    return (linear_f32_tc and not force_generic and a.dtype == torch.float32 and n % 32 == 0 and k % 32 == 0 and k >= 2048 and
+            n * k >= 1 << 20 and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
 def prefers_split(a: torch.Tensor, w: torch.Tensor) -> bool:
@@ -1356,8 +1373,8 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool
     accumulate=True adds the product into a float32 `out`.  cluster_slices=True: a product of at most 128 rows
     that stores bfloat16 cuts K into slices that meet in a thread-block cluster (every SM streams weights; without
     it such a product has one CTA per 128 output columns, which walks all of K).  bfloat16 products run on the tensor
-    cores (tcgen05) when K and the row stride of `a` are multiples of 8; float32 products, and
-    the sizes TMA cannot take, run on the SIMT kernel.
+    cores (tcgen05) when K and the row stride of `a` are multiples of 8; large float32 products run there as sums of exact
+    parts (_f32_tc_ok); other float32 products, and the sizes TMA cannot take, run on the SIMT kernel.
     `w` is taken for a loaded weight: float32 products of at most 16 rows and the tensor-core products begin to read it
     while earlier launches of this package still run, so none of those may be writing it.  (float32 products of more
     rows wait first.)"""
@@ -1394,6 +1411,11 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool
                 epi = EPI_ATOMIC_F32
         _call(lib, lib.tllm_linear_tc, _ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0), out.stride(0), epi, swap,
                                        splits, ctypes.c_float(0.0), _ptr(status_word(a.device)), _stream())
+        return
+    if _f32_tc_ok(a, w):
+        lib = build.load_library("linear_f32_tc")
+        _call(lib, lib.tllm_linear_f32_tc, _ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0), out.stride(0),
+                                           OUT_ACC if mode == OUT_ACC else OUT_F32, _cluster_slices(n, k), _ptr(status_word(a.device)), _stream())
         return
     lib = build.load_library("linear_generic")
     _call(lib, lib.tllm_linear_generic, _ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0), out.stride(0),
@@ -1773,7 +1795,7 @@ def sample(logits: torch.Tensor, work: torch.Tensor, temperature: torch.Tensor, 
                                 _ptr(seeds), _ptr(counters), _ptr(out), _ptr(status), _stream())
 
 
-ALL_LIBRARIES = ("elementwise", "linear_generic", "linear_tc", "attention_generic", "attention_prep", "recurrence",
+ALL_LIBRARIES = ("elementwise", "linear_generic", "linear_f32_tc", "linear_tc", "attention_generic", "attention_prep", "recurrence",
                  "linear_attention", "delta_rule", "head_linear", "window_attention", "attention_talk", "moe", "post_norm", "sampling")
 
 

@@ -24,7 +24,7 @@ BASE_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-shared", "-Xcompiler", "-fPIC"
 HEADERS = ["common.cuh", "per_device.h"]
 EXTRA_HEADERS = {"sampling": ["sampling_noalloc.h"], "attention_mma": ["attention_tiles.cuh"],
                  "attention_maps_mma": ["attention_tiles.cuh"], "attention_talk_mma": ["attention_tiles.cuh"],
-                 "linear_tc": ["tc_common.cuh"], "linear_generic": ["tc_common.cuh"], "delta_rule": ["tc_common.cuh"],
+                 "linear_tc": ["tc_common.cuh"], "linear_generic": ["tc_common.cuh"], "linear_f32_tc": ["tc_common.cuh"], "delta_rule": ["tc_common.cuh"],
                  "attention_tc": ["tc_common.cuh"], "attention_decode": ["tc_common.cuh"], "attention_generic": ["attention_route.h"],
                  "window_attention": ["window_attention.cuh"], "window_attention_mma": ["window_attention.cuh"]}   # per-source headers that enter the hash
 
