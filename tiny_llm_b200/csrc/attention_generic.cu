@@ -396,7 +396,7 @@ __device__ __forceinline__ float reduce_rows(const float (&in)[R], Op op, int la
 template <int OD, int R>
 struct RowsSmem {
   // Keys and values of a tile in buffers of their own, or values over the keys that have been multiplied.  Sixteen rows of up
-  // to 64 values: with one buffer two CTAs share an SM (97 KB of shared memory, 128 registers), and one computes while the
+  // to 64 values: with one buffer two CTAs share an SM (92 KB of shared memory, 128 registers), and one computes while the
   // other waits; with two buffers one CTA had an SM for itself (32 heads over 4 of 64, us: 131 tokens 24.1 -> 16.6, 509
   // 108.9 -> 76.1, 2,048 1,007 -> 698, 300 beside eight decoded ones 107.7 -> 90.9).
   static constexpr bool TWO = OD <= 2 && R < 16;
