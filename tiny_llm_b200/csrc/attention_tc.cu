@@ -32,14 +32,7 @@
 // softmax has read into registers by then): S/P of even tiles [0, 64), of odd tiles [64, 128), O
 // [128, 256).
 //
-// Latent attention (-DTLLM_HEAD_DIM=256 -DTLLM_VALUE_DIM=192: keys are a latent of 192 values and 64 rotated ones, values
-// the latent): four panels of keys, three of values; query tile, keys and values fill an SM's shared memory, so one CTA runs
-// alone, with keys (three stages) and values (two) in rings of their own, each fed by a warp: a key tile is free when its
-// scores are made, long before the product with its values.  Tensor memory: O at [128, 320) of 512 columns.
-// (A prompt of 1,777 tokens through four such layers of 16 heads: 5,445 -> 4,830 us a pass against the mma.sync kernel.)
-// A sink (a score per head that joins the softmax's denominator and has no value) is added at the end.
-//
-// Sizes: head size 64 or 128, or 256 with values of 192; heads per key/value head a power of two up to 128; page size 8, 16, 32
+// Sizes: head size 64 or 128; heads per key/value head a power of two up to 128; page size 8, 16, 32
 // or 64; no window.  Other cases run on the mma.sync kernels of attention_mma.cu.
 //
 // Reference counterpart: tiny_llm/ops/cuda/flash_attention.cu:338-442 (32-bit SIMT, one lane per
@@ -52,45 +45,39 @@
 #include "tc_common.cuh"
 
 #ifndef TLLM_HEAD_DIM
-#error "compile with -DTLLM_HEAD_DIM=64 or 128, or 256 and -DTLLM_VALUE_DIM=192"
-#endif
-#ifndef TLLM_VALUE_DIM
-#define TLLM_VALUE_DIM TLLM_HEAD_DIM
+#error "compile with -DTLLM_HEAD_DIM=64 or 128"
 #endif
 
 TLLM_DEFINE_LAST_ERROR
 
 namespace tllm {
 
-constexpr int HD = TLLM_HEAD_DIM, VD = TLLM_VALUE_DIM;
-static_assert((HD == VD && (HD == 64 || HD == 128)) || (HD == 256 && VD == 192), "rows of whole 128-byte swizzle rows that fit shared and tensor memory");
-constexpr int PANELS = HD / 64, VPANELS = VD / 64;  // panels of 64 columns (one swizzle row wide) of a query or key, of a value
-constexpr bool APART = HD > 128;                    // keys and values in rings of their own
+constexpr int HD = TLLM_HEAD_DIM;
+static_assert(HD == 64 || HD == 128, "a row of keys is one or two 128-byte swizzle rows");
+constexpr int PANELS = HD / 64;  // panels of 64 columns (one swizzle row wide) per operand
 constexpr int BM = 128;          // rows per CTA = MMA M
 constexpr int BNK = 64;          // keys per tile
-constexpr int K_STAGES = HD == 64 ? 4 : APART ? 3 : 2, V_STAGES = HD == 64 ? 4 : 2;
-constexpr int THREADS = APART ? 256 : 224;     // warp 0: TMA, warp 1: S = Q K^T + tensor memory, warps 2-5: softmax, warp 6: O += P V, APART: warp 7: TMA of the values
-constexpr int CTAS = APART ? 1 : 2;            // per SM
+constexpr int KV_STAGES = HD == 64 ? 4 : 2;
+constexpr int THREADS = 224;     // warp 0: TMA, warp 1: S = Q K^T + tensor memory, warps 2-5: softmax, warp 6: O += P V
 constexpr int UMMA_K = 16;
-constexpr int Q_BYTES = BM * HD * 2, K_BYTES = BNK * HD * 2, V_BYTES = BNK * VD * 2;
-constexpr int OFF_K = Q_BYTES, OFF_V = OFF_K + K_STAGES * K_BYTES;
-constexpr int OFF_BAR = OFF_V + V_STAGES * V_BYTES;
+constexpr int Q_BYTES = BM * HD * 2, K_BYTES = BNK * HD * 2, V_BYTES = BNK * HD * 2;
+constexpr int OFF_K = Q_BYTES, OFF_V = OFF_K + KV_STAGES * K_BYTES;
+constexpr int OFF_BAR = OFF_V + KV_STAGES * V_BYTES;
 constexpr int MAX_TABLE = 1024;                    // block-table entries kept in shared memory (longer tables are read from global)
 constexpr int OFF_TABLE = OFF_BAR + 160;
 constexpr int SMEM_TOTAL = OFF_TABLE + MAX_TABLE * 4 + 1024;   // + alignment slack
 constexpr int Q_PANEL = BM * 128, KV_PANEL = BNK * 128;   // bytes of one panel of Q / of a key or value tile
-constexpr uint32_t TMEM_COLS = APART ? 512 : 256;                // S of even tiles: columns [0, 64); of odd tiles: [64, 128); O: [128, 128 + HD);
+constexpr uint32_t TMEM_COLS = 256;                // S of even tiles: columns [0, 64); of odd tiles: [64, 128); O: [128, 128 + HD);
 // P (bfloat16 pairs): head size 64: even tiles [192, 224), odd tiles [224, 256); head size 128: over the tile's own S
 constexpr uint32_t TMEM_O = 2 * BNK, TMEM_P = HD == 64 ? TMEM_O + HD : 0, TMEM_P_STEP = HD == 64 ? BNK / 2 : BNK;
-static_assert(TMEM_O + VD <= TMEM_COLS && TMEM_P + TMEM_P_STEP + BNK / 2 <= TMEM_COLS, "S, O and P share 256 columns of tensor memory");
+static_assert(TMEM_O + HD <= TMEM_COLS && TMEM_P + TMEM_P_STEP + BNK / 2 <= TMEM_COLS, "S, O and P share 256 columns of tensor memory");
 constexpr float RESCALE_STEP = 8.f;
 
 struct TcAttnParams {
   const int* block_table;   // [R, max_blocks]
   const int* cu_q;          // [R + 1]
   const int* q_start;       // [R]: position of the request's first token in this step
-  __nv_bfloat16* out;       // [T, nq * VD]
-  const float* sink;        // [nq] or null
+  __nv_bfloat16* out;       // [T, nq * HD]
   int* status;
   int max_blocks, nq, nkv, page_size, tiles_per_req, n_requests;
   float scale_log2;         // scale * log2(e)
@@ -120,18 +107,17 @@ __device__ unsigned long long g_att_cycles[16];   // [8..15]: the MMA thread of 
 #define ATT_T(k)
 #endif
 
-__global__ void __launch_bounds__(THREADS, CTAS)
+__global__ void __launch_bounds__(THREADS, 2)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const TcAttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* q_full = bars;                       // [1]
-  uint64_t* k_full = bars + 1;                   // [K_STAGES]
-  uint64_t* v_full = k_full + K_STAGES;          // [V_STAGES]
-  uint64_t* kv_empty = v_full + V_STAGES;        // [V_STAGES]: the product with the values has read them (and the keys' stage, not APART)
-  uint64_t* k_empty = kv_empty + V_STAGES;       // [K_STAGES], APART: the scores are made
-  uint64_t* s_full = k_empty + (APART ? K_STAGES : 0);       // [2]: S of an even / odd tile is in tensor memory
+  uint64_t* k_full = bars + 1;                   // [KV_STAGES]
+  uint64_t* v_full = k_full + KV_STAGES;         // [KV_STAGES]
+  uint64_t* kv_empty = v_full + KV_STAGES;       // [KV_STAGES]
+  uint64_t* s_full = kv_empty + KV_STAGES;       // [2]: S of an even / odd tile is in tensor memory
   uint64_t* p_full = s_full + 2;                 // [2]: P of an even / odd tile is in tensor memory (its S has been read), O rescaled (one arrival per softmax warp)
   uint64_t* o_done = p_full + 2;                 // [2]: O holds an even / odd tile too, and its P buffer is free
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
@@ -150,8 +136,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int s = 0; s < K_STAGES; ++s) { mbar_init(&k_full[s], 1); if (APART) mbar_init(&k_empty[s], 1); }
-    for (int s = 0; s < V_STAGES; ++s) { mbar_init(&v_full[s], 1); mbar_init(&kv_empty[s], 1); }
+    for (int s = 0; s < KV_STAGES; ++s) { mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1); mbar_init(&kv_empty[s], 1); }
     mbar_init(&s_full[0], 1);
     mbar_init(&s_full[1], 1);
     mbar_init(&p_full[0], 4);
@@ -185,23 +170,21 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const int kv_end = start + q_len;                         // keys that exist once this step's are written
   const int n_tiles = row0 < rows_total ? (start + tok_hi) / BNK + 1 : 0;
 
-  if (warp == 0 || (APART && warp == 7)) {
+  if (warp == 0) {
     // ---------------- TMA producer.  A tile of 64 keys is up to eight pages, each a copy for K and one for V:
     // lane 2 g fetches the keys of the tile's page g, lane 2 g + 1 its values, so that the copies of a tile
     // are issued side by side (one thread issuing them all was the slowest part of the whole kernel).
     const int* table = p.block_table + (size_t)req * p.max_blocks;
     const int pages_per_tile = BNK / p.page_size;
     const uint32_t panel_page_bytes = (uint32_t)p.page_size * 128u;          // one page inside one panel
-    // lane = (page of the tile, keys or values, panel): COPIES per page, at most eight pages per tile (APART: warp 0 keys,
-    // warp 7 values)
-    constexpr int COPIES = APART ? PANELS : PANELS + VPANELS;
-    const bool mine_v = APART && warp == 7;
-    const int g = lane / COPIES, of_page = lane % COPIES;
-    const bool is_v = APART ? mine_v : of_page >= PANELS;
-    const int panel = !APART && is_v ? of_page - PANELS : of_page;
-    if (lane < PANELS && n_tiles > 0 && !mine_v) {
+    const uint32_t page_bytes = panel_page_bytes * PANELS;
+    // lane = (page of the tile, keys or values, panel): 2 * PANELS copies per page, at most eight pages per tile
+    const int g = lane / (2 * PANELS);
+    const bool is_v = (lane / PANELS) & 1;
+    const int panel = lane % PANELS;
+    if (lane < PANELS && n_tiles > 0) {
       if (lane == 0) mbar_expect_tx(q_full, Q_BYTES);
-      __syncwarp((1u << PANELS) - 1u);
+      __syncwarp(PANELS == 1 ? 1u : 3u);
       tma_load_3d(smem + lane * Q_PANEL, &map_q, lane * 64, kvh * group, tok0 + tok_lo, q_full);
     }
     __syncwarp();
@@ -211,11 +194,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     long long att_prev = clock64();
 #endif
     for (int i = 0; i < n_tiles; ++i) {
-      const int stages = mine_v ? V_STAGES : K_STAGES, s = i % stages;
+      const int s = i % KV_STAGES;
       ATT_T(5)   // producer: issuing
-      if (i >= stages) {
+      if (i >= KV_STAGES) {
         bool ok = true;
-        if (lane == 0) ok = mbar_wait(APART && !mine_v ? &k_empty[s] : &kv_empty[s], ((i / stages) & 1) ^ 1, abort_flag);
+        if (lane == 0) ok = mbar_wait(&kv_empty[s], ((i / KV_STAGES) & 1) ^ 1, abort_flag);
         if (!__shfl_sync(0xffffffffu, (int)ok, 0)) {
           if (lane == 0) { *abort_flag = 1; atomicExch(p.status, ERR_ATT_PRODUCER); }
           break;
@@ -225,11 +208,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       // this lane's page of keys [i * 64, i * 64 + 64), if it holds at least one existing key
       int page = -1;
       const int blk = i * pages_per_tile + g;
-      if (g < pages_per_tile && panel < (is_v ? VPANELS : PANELS) && blk < p.max_blocks && blk * p.page_size < kv_end) page = blk < MAX_TABLE ? table_s[blk] : table[blk];
-      const int n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0 && of_page == 0));
+      if (g < pages_per_tile && blk < p.max_blocks && blk * p.page_size < kv_end) page = blk < MAX_TABLE ? table_s[blk] : table[blk];
+      const int n_valid = __popc(__ballot_sync(0xffffffffu, page >= 0 && !is_v && panel == 0));
       if (lane == 0) {
-        if (!mine_v) mbar_expect_tx(&k_full[s], (uint32_t)(n_valid * PANELS) * panel_page_bytes);
-        if (!APART || mine_v) mbar_expect_tx(&v_full[s], (uint32_t)(n_valid * VPANELS) * panel_page_bytes);
+        mbar_expect_tx(&k_full[s], (uint32_t)n_valid * page_bytes);
+        mbar_expect_tx(&v_full[s], (uint32_t)n_valid * page_bytes);
       }
       __syncwarp();
       if (page >= 0) {
@@ -259,12 +242,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     long long att_prev = clock64();
 #endif
     for (int t = 0; t < n_tiles && ok; ++t) {
-      const int s = t % K_STAGES;
+      const int s = t % KV_STAGES;
       ATT_T(3)   // issuing
       if (t >= 2)   // tile t - 2: its S has been read, and its product has read the P buffer that the softmax of tile t will write
         ok = mbar_wait(&p_full[t & 1], ((t >> 1) - 1) & 1, abort_flag) && mbar_wait(&o_done[t & 1], ((t >> 1) - 1) & 1, abort_flag);
       ATT_T(1)   // waited for the S buffer
-      ok = ok && mbar_wait(&k_full[s], (t / K_STAGES) & 1, abort_flag);
+      ok = ok && mbar_wait(&k_full[s], (t / KV_STAGES) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
@@ -278,7 +261,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                        idesc_qk, k > 0 ? 1u : 0u);
         }
         umma_commit(&s_full[t & 1]);
-        if (APART) umma_commit(&k_empty[s]);
       }
       __syncwarp();
     }
@@ -289,10 +271,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     if (!ok && lane == 0 && !*abort_flag) { *abort_flag = 1; atomicExch(p.status, ERR_ATT_MMA); }
   } else if (warp == 6) {
     // ---------------- O += P V of tile i, when the softmax has written P (the same way: warp-wide loop, one lane issues)
-    const uint32_t idesc_pv = instr_desc_bf16(BM, VD, true);   // V as it lies: rows = keys (MN-major B)
+    const uint32_t idesc_pv = instr_desc_bf16(BM, HD, true);   // V as it lies: rows = keys (MN-major B)
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
     // head size 128: the values' second panel of 64 columns lies KV_PANEL bytes after the first
-    const uint32_t v_lo = smem_desc_sw128_lo(smem_u32(smem + OFF_V), VPANELS == 1 ? 16u : (uint32_t)KV_PANEL);
+    const uint32_t v_lo = smem_desc_sw128_lo(smem_u32(smem + OFF_V), PANELS == 1 ? 16u : (uint32_t)KV_PANEL);
     const uint32_t tmem_o = tmem_u + TMEM_O;
     bool ok = true;
 #ifdef TLLM_ATT_TIMING
@@ -301,11 +283,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     long long att_prev = clock64();
 #endif
     for (int i = 0; i < n_tiles; ++i) {
-      const int s = i % V_STAGES;
+      const int s = i % KV_STAGES;
       ATT_T(7)   // issuing
       ok = mbar_wait(&p_full[i & 1], (i >> 1) & 1, abort_flag);
       ATT_T(6)   // waited for P
-      ok = ok && mbar_wait(&v_full[s], (i / V_STAGES) & 1, abort_flag);
+      ok = ok && mbar_wait(&v_full[s], (i / KV_STAGES) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
@@ -347,7 +329,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     long long att_prev = clock64();
 #endif
     for (int i = 0; i < n_tiles; ++i) {
-      const int s = i % V_STAGES;
+      const int s = i % KV_STAGES;
       ok = mbar_wait(&s_full[i & 1], (i >> 1) & 1, abort_flag);   // (a wait that gave up is seen at this tile's vote below)
       tc_fence_after();
       ATT_T(0)   // waited for S
@@ -414,7 +396,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
-        for (int h = 0; h < VD; h += 32) {
+        for (int h = 0; h < HD; h += 32) {
           float o[32];
           tmem_ld32(t_o + h, o);
 #pragma unroll
@@ -425,12 +407,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       tmem_st_wait();
       ATT_T(5)   // O rescaled
       if (j0 + BNK > kv_end) {   // value rows past the last key hold whatever the page held: zero them
-        ok = mbar_wait(&v_full[s], (i / V_STAGES) & 1, abort_flag);
+        ok = mbar_wait(&v_full[s], (i / KV_STAGES) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         if (soft_tid < BNK && j0 + soft_tid >= kv_end) {
 #pragma unroll
-          for (int pn = 0; pn < VPANELS; ++pn) {
+          for (int pn = 0; pn < PANELS; ++pn) {
             uint4* vrow = reinterpret_cast<uint4*>(smem + OFF_V + s * V_BYTES + pn * KV_PANEL + soft_tid * 128);
 #pragma unroll
             for (int ch = 0; ch < 8; ++ch) vrow[ch] = make_uint4(0u, 0u, 0u, 0u);
@@ -455,18 +437,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       if (!*abort_flag) { *abort_flag = 1; atomicExch(p.status, ERR_ATT_SOFTMAX); }
     } else if (n_tiles > 0) {
       tc_fence_after();
-      float inv = 1.f / l_run;
-      if (p.sink != nullptr) {   // both terms of the denominator against the larger of the running maximum and the sink
-        const float sk = p.sink[kvh * group + grow % group] * 1.4426950408889634f, top = fmaxf(m_run, sk), f = ex2(m_run - top);
-        inv = f / fmaf(l_run, f, ex2(sk - top));
-      }
+      const float inv = 1.f / l_run;
       const size_t th = (size_t)(tok0 + grow / group) * p.nq + (size_t)(kvh * group + grow % group);
 #pragma unroll
-      for (int h = 0; h < VD; h += 32) {
+      for (int h = 0; h < HD; h += 32) {
         float o[32];
         tmem_ld32(t_o + h, o);   // warp-wide: rows that do not exist read too, and store nothing
         if (live) {
-          uint4* dst = reinterpret_cast<uint4*>(p.out + th * VD + h);
+          uint4* dst = reinterpret_cast<uint4*>(p.out + th * HD + h);
 #pragma unroll
           for (int ch = 0; ch < 4; ++ch) {
             uint4 v;
@@ -487,18 +465,18 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
 // ---------------------------------------------------------------- host side
 // Tensor maps are cached by what they describe; the step's buffers and the cache keep their addresses.
-static bool make_map_rows(CUtensorMap* map, const void* ptr, long long rows, int width, int box_rows) {
-  using Key = std::tuple<const void*, long long, int, int>;
+static bool make_map_rows(CUtensorMap* map, const void* ptr, long long rows, int box_rows) {
+  using Key = std::tuple<const void*, long long, int>;
   static std::map<Key, CUtensorMap> cache;
   static std::mutex mu;
-  const Key key(ptr, rows, width, box_rows);
+  const Key key(ptr, rows, box_rows);
   std::lock_guard<std::mutex> lock(mu);
   auto it = cache.find(key);
   if (it != cache.end()) { *map = it->second; return true; }
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)width * 2};
+  cuuint64_t dims[2] = {(cuuint64_t)HD, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)HD * 2};
   cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};   // one panel: a swizzle row of 128 bytes
   cuuint32_t elem[2] = {1, 1};
   if (fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
@@ -562,7 +540,7 @@ extern "C" int tllm_attention_tc_fits(int nq, int nkv, int hd, int page_size, in
 extern "C" int tllm_attention_tc(const void* q, int q_row_stride, const void* kcache, const void* vcache,
                                  long long cache_pages, const int* block_table, int max_blocks, const int* cu_q,
                                  const int* q_start, void* out, int n_tokens, int n_requests, int max_q_len, int nq,
-                                 int nkv, int hd, int page_size, float scale, const float* sink, int* status, void* stream) {
+                                 int nkv, int hd, int page_size, float scale, int* status, void* stream) {
   TLLM_REQUIRE(tllm_attention_tc_fits(nq, nkv, hd, page_size, 0), "attention_tc: %d heads, %d key/value heads, head size %d, page size %d "
                "(takes head size %d, a power-of-two group up to 128, pages of 8 to 64)", nq, nkv, hd, page_size, HD);
   TLLM_REQUIRE(n_tokens > 0 && n_requests > 0 && max_q_len > 0 && max_blocks > 0 && cache_pages > 0 && scale > 0.f && status != nullptr,
@@ -572,11 +550,11 @@ extern "C" int tllm_attention_tc(const void* q, int q_row_stride, const void* kc
   const int group = nq / nkv;
   CUtensorMap mq, mk, mv;
   const long long rows = cache_pages * nkv * page_size;
-  if (!make_map_q(&mq, q, n_tokens, nq, q_row_stride, group) || !make_map_rows(&mk, kcache, rows, HD, page_size) ||
-      !make_map_rows(&mv, vcache, rows, VD, page_size))
+  if (!make_map_q(&mq, q, n_tokens, nq, q_row_stride, group) || !make_map_rows(&mk, kcache, rows, page_size) ||
+      !make_map_rows(&mv, vcache, rows, page_size))
     TLLM_FAIL(TLLM_ERR_CUDA, "attention_tc: cuTensorMapEncodeTiled failed");
   TcAttnParams p;
-  p.block_table = block_table; p.cu_q = cu_q; p.q_start = q_start; p.out = (__nv_bfloat16*)out; p.sink = sink; p.status = status;
+  p.block_table = block_table; p.cu_q = cu_q; p.q_start = q_start; p.out = (__nv_bfloat16*)out; p.status = status;
   p.max_blocks = max_blocks; p.nq = nq; p.nkv = nkv; p.page_size = page_size;
   p.tiles_per_req = (int)(((long long)max_q_len * group + BM - 1) / BM);
   p.n_requests = n_requests;

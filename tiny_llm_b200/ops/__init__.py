@@ -1610,7 +1610,7 @@ def paged_attention(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, head_d
                 _ptr(qkv), qkv.stride(0), _ptr(k_cache), _ptr(v_cache), ctypes.c_longlong(k_cache.shape[0]),
                 _ptr(block_table), block_table.shape[1], _ptr(batch.cu_q), _ptr(batch.q_start), _ptr(out), t,
                 batch.num_requests, batch.max_q_len, num_heads, num_kv_heads, head_dim, page_size,
-                ctypes.c_float(scale), _ptr(None), _ptr(status_word(qkv.device)), _stream())
+                ctypes.c_float(scale), _ptr(status_word(qkv.device)), _stream())
             return
     if qkv.dtype == torch.bfloat16 and not force_generic and attention_decode_tma and head_dim in ATTENTION_TC_HEAD_DIMS and \
             not window and batch.max_q_len * group <= 16 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and \
@@ -1706,22 +1706,6 @@ def paged_attention_maps(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, m
             k_cache.shape[3] != key_dim or v_cache.stride(3) != 1 or v_cache.stride(2) != value_dim or \
             v_cache.shape[1] != num_kv_heads or v_cache.shape[3] != value_dim or k_cache.shape[2] != v_cache.shape[2]:
         raise KernelError("paged_attention_maps: shapes or dtypes do not fit")
-    if qkv.dtype == torch.bfloat16 and not force_generic and attention_tc and (key_dim, value_dim) in ATTENTION_TC_LATENT_DIMS and \
-            maps == 1 and not window and not chunk and rel is None and out.dtype == torch.bfloat16 and \
-            getattr(batch, "max_q_len", 0) * (num_heads // num_kv_heads) >= 128 and getattr(batch, "num_leading_decodes", 0) == 0 and \
-            scale > 0 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and k_cache.is_contiguous() and v_cache.is_contiguous() and \
-            k_cache.data_ptr() % 128 == 0 and v_cache.data_ptr() % 128 == 0 and out.data_ptr() % 16 == 0:
-        # Portions of prompts with latent keys and values: the tcgen05 kernel (four such layers of 16 heads in a prompt of 1,777
-        # tokens 820 us -> 200).  A step that brings decoded tokens first stays on the kernel below, whose CTAs have 64 rows
-        # instead of 128: here a decoded token's 16 rows would leave seven eighths of a tile empty.
-        lib = build.load_library("attention_tc", flags=(f"-DTLLM_HEAD_DIM={key_dim}", f"-DTLLM_VALUE_DIM={value_dim}"))
-        if lib.tllm_attention_tc_fits(num_heads, num_kv_heads, key_dim, k_cache.shape[2], 0):
-            _call(lib, lib.tllm_attention_tc,
-                  _ptr(qkv), qkv.stride(0), _ptr(k_cache), _ptr(v_cache), ctypes.c_longlong(k_cache.shape[0]),
-                  _ptr(block_table), block_table.shape[1], _ptr(batch.cu_q), _ptr(batch.q_start), _ptr(out), t,
-                  batch.num_requests, batch.max_q_len, num_heads, num_kv_heads, key_dim, k_cache.shape[2],
-                  ctypes.c_float(scale), _ptr(sink), _ptr(status_word(qkv.device)), _stream())
-            return
     few = getattr(batch, "max_q_len", 0) == 1 and t * num_heads * maps <= attention_maps_decode_pairs
     if qkv.dtype == torch.bfloat16 and not force_generic and attention_maps_tc and \
             (rel is None or rel_log2 is not None) and not few and scale > 0 and key_dim % 16 == 0 and value_dim % 16 == 0 and 16 <= key_dim <= 256 and 16 <= value_dim <= 256 and \
@@ -1817,7 +1801,6 @@ ALL_LIBRARIES = ("elementwise", "linear_generic", "linear_f32_tc", "linear_tc", 
 
 ATTENTION_HEAD_DIMS = (16, 32, 48, 64, 128)   # head sizes `build_all` compiles ahead; others compile on first use
 ATTENTION_TC_HEAD_DIMS = (64, 128)            # head sizes the tcgen05 prompt-attention kernel is written for
-ATTENTION_TC_LATENT_DIMS = ((256, 192),)      # ... and (key size, value size) of latent attention
 ATTENTION_MAPS_DIMS = ((64, 128), (128, 128), (256, 192))           # (key size, value size) pairs of the multi-map kernel compiled ahead
 
 
@@ -1834,8 +1817,6 @@ def build_all(verbose: bool = True):
               for hd in ATTENTION_HEAD_DIMS]
     paths += [build.compile_library("attention_tc", flags=(f"-DTLLM_HEAD_DIM={hd}",), verbose=verbose)
               for hd in ATTENTION_TC_HEAD_DIMS]
-    paths += [build.compile_library("attention_tc", flags=(f"-DTLLM_HEAD_DIM={kd}", f"-DTLLM_VALUE_DIM={vd}"), verbose=verbose)
-              for kd, vd in ATTENTION_TC_LATENT_DIMS]
     paths += [build.compile_library("attention_decode", flags=(f"-DTLLM_HEAD_DIM={hd}",), verbose=verbose)
               for hd in ATTENTION_TC_HEAD_DIMS]
     paths += [build.compile_library("attention_maps_mma", flags=(f"-DTLLM_HEAD_DIM={kd}", f"-DTLLM_VALUE_DIM={vd}"), verbose=verbose)
