@@ -16,13 +16,13 @@ def ops():
 
 
 def bound(a, w):
-    """What the sums may be away from 64 bits: the three partial products left out (2^-24 each of |a w| at most), three
-    accumulators that add 16 products at a time (4 + 8 + 12 additions per block of 64, of which the last twenty are 2^-7
-    smaller) with at most two units of truncation of the block's |a w| each, and three additions per block to the running
-    sum."""
+    """What the sums may be away from 64 bits, in sizes |a w| added up: the product left out (2^-34); the large accumulator, four
+    additions of 16 products per block of 64 with at most two units of truncation of the block's sizes each; the small ones,
+    2^-8 of the sizes (or less), with eight additions per 16 values of k; an addition to the running sum per block, two for the
+    small ones and three for the slices."""
     k = a.shape[1]
     size = a.double().abs() @ w.double().abs().T
-    return (3 * 2.0 ** -24 + (4 + 20 * 2.0 ** -7) * 2.0 ** -22 + (3 * math.ceil(k / 64) + 8) * 2.0 ** -24) * size
+    return (2.0 ** -34 + 4 * 2.0 ** -22 + 8 * math.ceil(k / 16) * 2.0 ** -30 + (math.ceil(k / 64) + 5) * 2.0 ** -24) * size
 
 
 @pytest.mark.parametrize("n,k", [(512, 2048), (4128, 2048), (32, 32768), (544, 2080), (2048, 3040), (32000, 2048), (1056, 2208)])
@@ -43,6 +43,43 @@ def test_rows_of_every_count_are_near_64_bits_and_depend_on_no_other_row(ops, n,
         assert torch.equal(acc, whole[:m] + 0.5), m
     ops.check_status()
     assert bool(((whole - want).abs() <= most).all())
+
+
+def test_a_single_product_is_as_near_as_one_rounding(ops):
+    """Rows of one value each: eight partial products leave 2^-34 out, and the sum is rounded once (2^-24).  With parts that are cut
+    instead of rounded the first pair is 4.7e-7 off."""
+    g = torch.Generator(device=DEV).manual_seed(1)
+    n, k = 512, 2048
+    for m in (16, 200):
+        a, w = torch.zeros(m, k, device=DEV), torch.zeros(n, k, device=DEV)
+        a[:, 77] = torch.randn(m, generator=g, device=DEV)
+        w[:, 77] = torch.randn(n, generator=g, device=DEV)
+        a[0, 77] = w[0, 77] = 1 + 2.0 ** -7 - 2.0 ** -23
+        out = torch.empty(m, n, device=DEV)
+        ops.linear(a, w, out)
+        want = a[:, 77:78].double() @ w[:, 77:78].double().T
+        assert bool(((out - want).abs() <= want.abs() * (2.0 ** -24 + 2.0 ** -34)).all())
+    ops.check_status()
+
+
+@pytest.mark.parametrize("n", [512, 32000])
+@pytest.mark.parametrize("values", [1, 2, 4, 8, 16])
+def test_rows_of_few_values_are_as_near_as_one_chain_of_fmaf(ops, n, values, monkeypatch):
+    """A chain rounds once per value.  The tensor cores' sums are rounded once per block with values and once more per slice with
+    values (n = 512: eight slices), so two to four values in slices of their own come out up to a sixth further off."""
+    g = torch.Generator(device=DEV).manual_seed(values + n)
+    m, k, away = 400, 2048, {}
+    a = torch.zeros(m, k, device=DEV)
+    where = torch.rand(m, k, generator=g, device=DEV).argsort(1)[:, :values]
+    a.scatter_(1, where, torch.randn(m, values, generator=g, device=DEV))
+    w = torch.randn(n, k, generator=g, device=DEV)
+    want, size = a.double() @ w.double().T, (a.double().abs() @ w.double().abs().T).clamp_min(1e-30)
+    for tc in (True, False):
+        monkeypatch.setattr(ops, "linear_f32_tc", tc)
+        out = torch.empty(m, n, device=DEV)
+        ops.linear(a, w, out)
+        away[tc] = float(((out - want) / size).square().mean().sqrt())
+    assert away[True] <= away[False] * 1.2, away
 
 
 @pytest.mark.parametrize("n,k", [(2048, 2048), (2048, 5632), (11264, 2048)])

@@ -1,13 +1,16 @@
 // float32 products C[M,N] = A[M,K] . W[N,K]^T on the 5th-generation tensor cores, for the 32-bit path: every factor is
-// the exact sum of three bfloat16 values (24 bits of mantissa in three times 8: x = hi + mid + lo, each the truncation of
-// what is left), and a product is the sum of the six partial products above 2^-24 of it,
-//   hi hi | hi mid + mid hi | hi lo + mid mid + lo hi,
-// each group in a tensor-memory accumulator of its own.
+// the sum of three bfloat16 values (24 bits of mantissa in three times 8: x = hi + mid + lo, each what is left rounded to
+// nearest, so that mid is at most 2^-8 of x, lo 2^-17, and both have either sign), and a product is the sum of eight
+// partial products: all but lo lo, which is below 2^-33 of it.  (Parts cut instead of rounded have the sign of x and up to
+// twice the size; with them and six products a single product was up to 4.7e-7 off, an fmaf is 6.0e-8 at most.)
 //
-// The tensor cores add with less care than an fmaf, so no accumulator lives long: after every 64 values of k the three
-// are read back and added, in that order, to 32-bit sums in registers, and start again from nothing.  (Relative error
-// against 64 bits, 2-norm, normal operands, here / one chain of fmaf: K = 2,048 1.4e-7 to 2.1e-7 / 8.1e-7, K = 5,632
-// 1.7e-7 / 1.3e-6.)
+// The tensor cores cut what an fmaf rounds, so the accumulator of hi hi does not live long: after every 64 values of k
+// it is read back, added to 32-bit sums in registers, and starts again from nothing.  The seven small products, 2^-8 of the
+// whole and less, share accumulators that live through a slice of K and join its sum once: what is cut there is 2^-32.
+// Relative error against 64 bits, 2-norm, normal operands, here / one chain of fmaf: K = 2,048 0.9e-7 to 1.3e-7 / 8.1e-7,
+// K = 5,632 1.1e-7 / 1.3e-6.  Rows of few values (rms in sizes |a w| added up, 1 / 2 / 4 / 8 / 16 of 2,048 values): 2.5e-8, 2.1,
+// 1.8, 1.4, 1.3e-8 in one slice of K, 2.6e-8, 3.0, 2.9, 2.5, 1.9e-8 in eight (a rounding more per slice), the chain 2.5e-8, 2.6,
+// 2.7, 2.7, 2.9e-8.
 //
 // The sums' order is a function of N and K alone -- k ascending in blocks of 64 within each of `slices` runs of blocks, the
 // runs added in pairs, pairs of pairs and so on -- whatever M is and whichever shape of the kernel takes it, so a row's
@@ -38,20 +41,20 @@ constexpr int KS = 32;               // values of k per step: one 128-byte row o
 constexpr int ROW_BYTES = 128;
 constexpr int OUT_STORE = 1, OUT_ADD = 2;
 
-template <int BN_, bool CONCAT_, int RAW_, int STAGES_, int DBUF_, int W_GROUPS_, int T_GROUPS_, int T_WARPS_, int E_COLS_, int CTAS_,
+template <int BN_, int RAW_, int STAGES_, int DBUF_, int W_GROUPS_, int T_GROUPS_, int T_WARPS_, int E_COLS_, int CTAS_,
           bool PAIRS_ = false, int REGS_ = 0>
 struct Shape {
   static constexpr int BN = BN_;               // rows of A per CTA
-  static constexpr bool CONCAT = CONCAT_;      // the three accumulators side by side as one MMA of 3 BN columns
   static constexpr int RAW = RAW_;             // steps of float32 in flight
   static constexpr int STAGES = STAGES_;       // split steps in flight
-  static constexpr int DBUF = DBUF_;           // sets of accumulators
+  static constexpr int DBUF = DBUF_;           // accumulators of hi hi
   static constexpr int W_GROUPS = W_GROUPS_;   // groups of four warps that split weights, step by step in turn
   static constexpr int T_GROUPS = T_GROUPS_, T_WARPS = T_WARPS_;   // groups of warps that split rows of A, in turn as well
   static constexpr int E_COLS = E_COLS_;       // columns per warp of the running sums
   static constexpr int CTAS = CTAS_;           // per SM
   static constexpr bool PAIRS = PAIRS_;        // may walk two slices
   static constexpr int REGS = REGS_;           // > 0: registers of a summing thread; the others give theirs up (whole warpgroups)
+  static constexpr int S_READ = PAIRS || E_COLS > 16 ? 8 : 16;     // columns of small products read at a time (registers)
   static constexpr int E_WARPS = 4 * (BN / E_COLS);
   static constexpr int W0 = REGS > 0 ? 4 : 2, T0 = W0 + 4 * W_GROUPS, E0 = T0 + T_GROUPS * T_WARPS, WARPS = E0 + E_WARPS, THREADS = WARPS * 32;
   static constexpr int W_RAW = ROWS * ROW_BYTES, T_RAW = BN * ROW_BYTES, RAW_BYTES = W_RAW + T_RAW;
@@ -59,17 +62,18 @@ struct Shape {
   static constexpr int B_SLOTS = (STAGES + 1) / 2;
   static constexpr int B_OFFSET = RAW * RAW_BYTES;
   static constexpr int BAR_OFFSET = B_OFFSET + B_SLOTS * B_SLOT;
-  static constexpr int BARS = 2 * RAW + 2 * STAGES + 6 + 1;
+  static constexpr int BARS = 2 * RAW + 2 * STAGES + 2 * DBUF + 3;
   static constexpr int SMEM = BAR_OFFSET + BARS * 8 + 16 + 1024;   // + alignment slack
-  static constexpr int A_COLS = 3 * (KS / 2);                      // tensor-memory columns of a split weight step
-  static constexpr int A_BASE = DBUF * 3 * BN;
+  // tensor memory: the small products' two accumulators, those of hi hi, split weight steps
+  static constexpr int A_COLS = 3 * (KS / 2);
+  static constexpr int D_BASE = 2 * BN, A_BASE = D_BASE + DBUF * BN;
   static constexpr int TMEM_USED = A_BASE + STAGES * A_COLS;
   static constexpr int TMEM_COLS = TMEM_USED <= 256 ? 256 : 512;
   // (a split of registers draws on what the block was launched with)
   static constexpr int LAUNCH_REGS = 65536 / THREADS / 8 * 8, OTHER_REGS = 48;
   static_assert(REGS == 0 || (E0 % 4 == 0 && E_WARPS % 4 == 0 && E_WARPS * 32 * REGS + E0 * 32 * OTHER_REGS <= THREADS * LAUNCH_REGS), "registers");
   static_assert(TMEM_USED <= 512 && CTAS * TMEM_COLS <= 512, "tensor memory");
-  static_assert(CONCAT ? 3 * BN <= 256 : DBUF == 1, "one MMA's columns; one set of accumulators that are drained in turn");
+  static_assert(2 * BN <= 256 && DBUF <= 2, "one MMA's columns; accumulators");
   static_assert(BN * ROWS * 4 <= B_OFFSET, "the sums are parked where the float32 steps were");
   static_assert(BN * (KS / 8) % (T_WARPS * 32) == 0, "whole tasks per lane");
   // A role waits by parity, so a slot's use before the one it waits for must not be two behind: either the slot's uses are
@@ -81,6 +85,10 @@ struct Shape {
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t* r) {   // (tmem_ld_wait() before the values are used)
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ float4 ld_shared4(uint32_t at) {
   float4 v;
@@ -102,15 +110,13 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Two neighbouring values as three pairs of bfloat16, the first of a pair in the low half.  Both subtractions are exact.
+// Two neighbouring values as three pairs of bfloat16, the first of a pair in the low half.  All four subtractions are exact.
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
-  hi = __byte_perm(xb, yb, 0x7632);
-  const float rx = x - __uint_as_float(xb & 0xffff0000u), ry = y - __uint_as_float(yb & 0xffff0000u);
-  const uint32_t rxb = __float_as_uint(rx), ryb = __float_as_uint(ry);
-  mid = __byte_perm(rxb, ryb, 0x7632);
-  const float sx = rx - __uint_as_float(rxb & 0xffff0000u), sy = ry - __uint_as_float(ryb & 0xffff0000u);
-  lo = __byte_perm(__float_as_uint(sx), __float_as_uint(sy), 0x7632);
+  auto pair = [](float a, float b) { const __nv_bfloat162 h = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const uint32_t*>(&h); };
+  hi = pair(x, y);
+  const float rx = x - __uint_as_float(hi << 16), ry = y - __uint_as_float(hi & 0xffff0000u);
+  mid = pair(rx, ry);
+  lo = pair(rx - __uint_as_float(mid << 16), ry - __uint_as_float(mid & 0xffff0000u));
 }
 
 // One element as the other kernels of the 32-bit path make it.
@@ -132,9 +138,11 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   uint64_t* raw_empty = raw_full + S::RAW;
   uint64_t* split_full = raw_empty + S::RAW;
   uint64_t* split_empty = split_full + S::STAGES;
-  uint64_t* d_full = split_empty + S::STAGES;      // [3]: concat: the set's; else one per accumulator
-  uint64_t* d_empty = d_full + 3;
-  uint64_t* end_bar = d_empty + 3;
+  uint64_t* d_full = split_empty + S::STAGES;      // [DBUF]: a block's hi hi lies in tensor memory / has been read
+  uint64_t* d_empty = d_full + S::DBUF;
+  uint64_t* s_full = d_empty + S::DBUF;            // a slice's small products lie in tensor memory / have been read
+  uint64_t* s_empty = s_full + 1;
+  uint64_t* end_bar = s_empty + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(end_bar + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
@@ -145,13 +153,16 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   const int blocks = max(0, min(all_blocks - block0, slices_per_cta * blocks_per_slice));
   const int steps = 2 * blocks;                    // (an odd last step reads zeros past the end of K)
   const int k0 = block0 * 2 * KS;
+  auto ends_slice = [&](int block) { return block == blocks - 1 || (S::PAIRS && block == blocks_per_slice - 1); };
 
   if (threadIdx.x == 0) {
     tma_prefetch_map(&map_w);
     tma_prefetch_map(&map_a);
     for (int s = 0; s < S::RAW; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 4 + S::T_WARPS); }
     for (int s = 0; s < S::STAGES; ++s) { mbar_init(&split_full[s], 4 + S::T_WARPS); mbar_init(&split_empty[s], 1); }
-    for (int s = 0; s < 3; ++s) { mbar_init(&d_full[s], 1); mbar_init(&d_empty[s], S::E_WARPS); }
+    for (int s = 0; s < S::DBUF; ++s) { mbar_init(&d_full[s], 1); mbar_init(&d_empty[s], S::E_WARPS); }
+    mbar_init(s_full, 1);
+    mbar_init(s_empty, S::E_WARPS);
     mbar_init(end_bar, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -197,57 +208,46 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
       const uint32_t b_lo0 = smem_desc_sw128_lo(base + S::B_OFFSET);
       constexpr uint32_t PART = (uint32_t)(BN * ROW_BYTES) >> 4;   // from hi to mid to lo, in descriptor units
+      const uint32_t two = instr_desc_bf16(ROWS, 2 * BN), one = instr_desc_bf16(ROWS, BN);
       bool ok = true;
       for (int i = 0; i < steps; ++i) {
-        const int s = i % S::STAGES, half = i & 1, block = i >> 1;
-        ok = __all_sync(0xffffffffu, mbar_wait(&split_full[s], (i / S::STAGES) & 1, abort_flag));
+        const int s = i % S::STAGES, half = i & 1, block = i >> 1, set = block % S::DBUF;
+        const bool second = S::PAIRS && half == 0 && block == blocks_per_slice, fresh = i == 0 || second;
+        ok = mbar_wait(&split_full[s], (i / S::STAGES) & 1, abort_flag);
+        if (second) ok = ok && mbar_wait(s_empty, 0, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t at = tm + S::A_BASE + s * S::A_COLS;
+        const uint32_t at = tm + S::A_BASE + s * S::A_COLS, d = tm + S::D_BASE + set * BN;
         const uint32_t bt = b_lo0 + (uint32_t)((s >> 1) * S::B_SLOT >> 4) + (uint32_t)((s & 1) * 64 >> 4);
-        if (S::CONCAT) {
-          const int set = block % S::DBUF;
-          if (half == 0) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&d_empty[set], ((block / S::DBUF) & 1) ^ 1, abort_flag));
-            if (!ok) break;
-            tc_fence_after();
-          }
-          const uint32_t d = tm + set * 3 * BN;
-          const uint32_t i3 = instr_desc_bf16(ROWS, 3 * BN), i2 = instr_desc_bf16(ROWS, 2 * BN), i1 = instr_desc_bf16(ROWS, BN);
-          if (elect_one()) {
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const uint32_t more = (half > 0 || q > 0) ? 1u : 0u;
-              umma_bf16_ts_lo(d, at + q * 8, bt + q * 2, i3, more);                    // hi x [hi | mid | lo]
-              umma_bf16_ts_lo(d + BN, at + 16 + q * 8, bt + q * 2, i2, 1u);            // mid x [hi | mid]
-              umma_bf16_ts_lo(d + 2 * BN, at + 32 + q * 8, bt + q * 2, i1, 1u);        // lo x [hi]
-            }
-            umma_commit(&split_empty[s]);
-            if (half == 1) umma_commit(&d_full[set]);
-          }
+        auto small = [&](int q) {
+          umma_bf16_ts_lo(tm, at + q * 8, bt + PART + q * 2, two, fresh && q == 0 ? 0u : 1u);   // hi x [mid | lo]
+          umma_bf16_ts_lo(tm, at + 16 + q * 8, bt + q * 2, two, 1u);                            // mid x [hi | mid]
+          umma_bf16_ts_lo(tm, at + 32 + q * 8, bt + q * 2, two, 1u);                            // lo x [hi | mid]
+          umma_bf16_ts_lo(tm, at + 16 + q * 8, bt + 2 * PART + q * 2, one, 1u);                 // mid x [lo]
+        };
+        auto large = [&](int q) { umma_bf16_ts_lo(d, at + q * 8, bt + q * 2, one, half > 0 || q > 0 ? 1u : 0u); };   // hi x [hi]
+        // One accumulator of hi hi: the small products of a block's first half are made while it is read out.  Two: it has been
+        // read by now, and one run of ten products is the faster (eight rows of A, us, two runs / one: 11,264 x 2,048 23.2 /
+        // 22.3, 2,048 x 5,632 17.0 / 16.2, 2,048 x 2,048 8.6 / 8.3).
+        const bool apart = S::DBUF == 1 && half == 0;
+        if (apart) {
+          if (elect_one()) { small(0); small(1); }
           __syncwarp();
-        } else {
-          const uint32_t idesc = instr_desc_bf16(ROWS, BN);
-#pragma unroll
-          for (int g = 0; g < 3; ++g) {    // accumulator g: the parts whose numbers add up to g
-            if (half == 0) {
-              ok = ok && __all_sync(0xffffffffu, mbar_wait(&d_empty[g], (block & 1) ^ 1, abort_flag));
-              if (!ok) break;
-              tc_fence_after();
-            }
-            if (elect_one()) {
-#pragma unroll
-              for (int q = 0; q < 2; ++q)
-#pragma unroll
-                for (int p = 0; p <= g; ++p)      // part p of the weights, part g - p of the rows of A
-                  umma_bf16_ts_lo(tm + g * BN, at + p * 16 + q * 8, bt + (g - p) * PART + q * 2, idesc, (half > 0 || q > 0 || p > 0) ? 1u : 0u);
-              if (g == 2) umma_commit(&split_empty[s]);
-              if (half == 1) umma_commit(&d_full[g]);
-            }
-            __syncwarp();
-          }
-          if (!ok) break;
         }
+        if (half == 0) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&d_empty[set], ((block / S::DBUF) & 1) ^ 1, abort_flag));
+          if (!ok) break;
+          tc_fence_after();
+        }
+        if (elect_one()) {
+          if (!apart) { large(0); small(0); large(1); small(1); }
+          else { large(0); large(1); }
+          umma_commit(&split_empty[s]);
+          if (half == 1) umma_commit(&d_full[set]);
+          if (half == 1 && ends_slice(block)) umma_commit(s_full);
+        }
+        __syncwarp();
       }
       if (!ok && lane == 0) { *abort_flag = 1; atomicExch(status, ERR_FT_MMA); }
       // nothing is in flight when the tensor memory goes back
@@ -272,6 +272,10 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
           float4 v[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) v[j] = ld_shared4(src + (uint32_t)(((q * 4 + j) ^ (row & 7)) << 4));
+          if (q == 1) {      // the float32 values are in registers
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&raw_empty[r]);
+          }
           uint32_t hi[8], mid[8], lo[8];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -285,7 +289,7 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) { mbar_arrive(&raw_empty[r]); mbar_arrive(&split_full[s]); }
+        if (lane == 0) mbar_arrive(&split_full[s]);
       }
       if (!ok && lane == 0) { *abort_flag = 1; atomicExch(status, ERR_FT_SPLIT); }
     } else if (warp >= S::T0) {
@@ -340,27 +344,36 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
 #pragma unroll
         for (int c = 0; c < S::E_COLS; ++c) { first[S::PAIRS ? c : 0] = acc[c]; acc[c] = 0.f; }
       }
-      const int set = S::CONCAT ? b % S::DBUF : 0;
+      const int set = b % S::DBUF;
+      ok = __all_sync(0xffffffffu, mbar_wait(&d_full[set], (b / S::DBUF) & 1, abort_flag));
+      if (!ok) break;
+      tc_fence_after();
 #pragma unroll
-      for (int g = 0; g < 3; ++g) {
-        if (!S::CONCAT || g == 0) {
-          const int bar = S::CONCAT ? set : g;
-          ok = __all_sync(0xffffffffu, mbar_wait(&d_full[bar], (S::CONCAT ? b / S::DBUF : b) & 1, abort_flag));
-          if (!ok) break;
-          tc_fence_after();
-        }
+      for (int c = 0; c < S::E_COLS; c += 16) {
+        float v[16];
+        tmem_ld16(t_at + S::D_BASE + set * BN + c, v);
 #pragma unroll
-        for (int c = 0; c < S::E_COLS; c += 16) {
-          float v[16];
-          tmem_ld16(t_at + (S::CONCAT ? set * 3 * BN : 0) + g * BN + c, v);
+        for (int j = 0; j < 16; ++j) acc[c + j] += v[j];
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&d_empty[set]);
+      if (ends_slice(b)) {
+        ok = __all_sync(0xffffffffu, mbar_wait(s_full, b >= blocks_per_slice ? 1 : 0, abort_flag));
+        if (!ok) break;
+        tc_fence_after();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) acc[c + j] += v[j];
+        for (int c = 0; c < S::E_COLS; c += S::S_READ) {
+          uint32_t u[S::S_READ], v[S::S_READ];
+#pragma unroll
+          for (int j = 0; j < S::S_READ; j += 8) { tmem_ld8_issue(t_at + c + j, u + j); tmem_ld8_issue(t_at + BN + c + j, v + j); }
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < S::S_READ; ++j) acc[c + j] += __uint_as_float(u[j]) + __uint_as_float(v[j]);
         }
-        if (!S::CONCAT || g == 2) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&d_empty[S::CONCAT ? set : g]);
-        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_empty);
       }
     }
     if (!ok && lane == 0) { *abort_flag = 1; atomicExch(status, ERR_FT_SUMS); }
@@ -462,17 +475,19 @@ static int launch_shape(const float* a, const float* w, float* out, int m, int n
   return launch_mode<S, OUT_STORE>(a, w, out, m, n, k, lda, ldo, slices, early, status, s, sms);
 }
 
-// Which shape: the smallest that holds the rows.  Few rows are bound by the weights from memory, 5 TB/s of them with two CTAs on
-// every SM, and by 7 us that a launch takes whatever it multiplies; many by the read-out of the accumulators beside the MMAs
-// (more splitting warps changed nothing; 96 rows per CTA with four stages took 57 us instead of 64 with one slice of 2,560
-// x 2,048 x 509, but 105 instead of 91 with eight).  us, m = 1 / 8 / 64 / 509, one chain of fmaf per element: 2,560 x 2,048
-// 8.5 / 14.2 / 56 / 146, 2,048 x 2,048 8.1 / 13.7 / 38 / 103, 11,264 x 2,048 23.4 / 28.3 / 105 / 461, 2,048 x 5,632 19.7 /
-// 34.4 / 100 / 277; here 9.2 / 9.5 / 16 / 66, 9.0 / 9.4 / 22 / 45, 24.8 / 24 / 48 / 178, 17.7 / 17.3 / 37 / 93.
-//                    BN  concat RAW STAGES DBUF W_GROUPS T_GROUPS T_WARPS E_COLS CTAS PAIRS REGS
-using Shape16 = Shape<16, true, 5, 3, 2, 2, 2, 1, 16, 2>;
-using Shape128 = Shape<128, false, 5, 2, 1, 1, 1, 4, 64, 1, true, 168>;
-using Shape32 = Shape<32, true, 4, 3, 1, 2, 1, 2, 32, 2>;
-using Shape64 = Shape<64, true, 6, 2, 2, 2, 1, 4, 32, 1, true>;
+// Which shape: the smallest that holds the rows.  Few rows are bound by the weights from memory, up to 6 TB/s of them with two
+// CTAs on every SM, and by what a launch takes whatever it multiplies (7.8 us for 2,048 x 2,048, whose weights take 2.6); many by
+// the tensor cores and the read-out beside them.  us, m = 1 / 8 / 64 / 509, launches in a graph, weights from memory, one chain of
+// fmaf per element: 2,560 x 2,048 7.8 / 13.4 / 55 / 144, 2,048 x 2,048 7.5 / 12.9 / 37 / 101, 11,264 x 2,048 23.1 / 27.3 / 103 /
+// 458, 2,048 x 5,632 18.6 / 33.6 / 99 / 274; here 8.2 / 8.4 / 15.5 / 62, 7.8 / 8.2 / 20.9 / 42, 21.9 / 22.3 / 48 / 162, 15.6 /
+// 16.0 / 37 / 83.  With six products and parts that are cut: 8.2 / 8.6 / 14.7 / 64, 8.1 / 8.4 / 20.6 / 43, 21.9 / 22.3 / 46 / 174,
+// 16.0 / 16.3 / 35 / 89: the two products more cost 33 to 64 rows 1 to 6 %.
+// Other forms of Shape64: weights split by two groups of warps 2 to 3 % slower, three or four stages 1 to 4 %.
+//                    BN RAW STAGES DBUF W_GROUPS T_GROUPS T_WARPS E_COLS CTAS PAIRS REGS
+using Shape16 = Shape<16, 5, 3, 2, 2, 2, 1, 16, 2>;
+using Shape128 = Shape<128, 5, 2, 1, 1, 1, 4, 64, 1, true, 168>;
+using Shape32 = Shape<32, 4, 2, 2, 2, 1, 2, 32, 2>;
+using Shape64 = Shape<64, 6, 2, 2, 1, 1, 4, 32, 1, true>;
 
 }  // namespace tllm
 
