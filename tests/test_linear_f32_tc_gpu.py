@@ -97,6 +97,27 @@ def test_no_further_from_64_bits_than_one_chain_of_fmaf(ops, n, k, monkeypatch):
         assert away[True] <= away[False], away
 
 
+@pytest.mark.parametrize("m", [8, 40, 130])
+def test_operands_of_every_size_are_split_exactly(ops, m):
+    """Rows of 1e-25 to the smallest subnormal numbers against weights of 1e-6 to 1e20, and rows near the largest numbers against
+    small weights: the bound is the same, beside the last place of a subnormal result.  (The largest are made as chains of
+    fmaf, 2^-24 per value.)"""
+    g = torch.Generator(device=DEV).manual_seed(m)
+    n, k = 1024, 2048
+    a, w = torch.randn(m, k, generator=g, device=DEV), torch.randn(n, k, generator=g, device=DEV)
+    sizes = torch.tensor([1e-25, 1e-30, 1e-33, 1e-35, 1e-36, 2e-38, 1e-40, 1e20, 1e30, 1e32, 1e36], dtype=torch.float64, device=DEV)
+    a = (a.double() * sizes[torch.arange(m, device=DEV) % len(sizes)][:, None]).float()
+    w = w * torch.tensor([1.0, 1e-6, 1e20, 1e-3], device=DEV)[torch.arange(n, device=DEV) % 4][:, None]
+    out = torch.empty(m, n, device=DEV)
+    ops.linear(a, w, out)
+    want = a.double() @ w.double().T
+    size = a.double().abs() @ w.double().abs().T
+    here = size < 1e38                     # (no partial sum of a chain overflows)
+    most = torch.where(a.abs().amax(1, keepdim=True) > 1e19, size * k * 2.0 ** -24, bound(a, w)) + 2.0 ** -149
+    assert bool(((out - want).abs() <= most)[here].all()) and int(here.sum()) > m * n // 2
+    ops.check_status()
+
+
 def test_operands_that_are_not_finite_give_what_one_chain_of_fmaf_gives(ops, monkeypatch):
     g = torch.Generator(device=DEV).manual_seed(3)
     n, k = 1024, 2048

@@ -24,8 +24,8 @@
 // The slices of a tile, or pairs of slices that a CTA walks one after the other, are a thread-block cluster that adds its sums
 // through distributed shared memory.
 //
-// A sum that is not finite (an operand was infinite or NaN, or the sums overflowed) is computed again as the other
-// kernels of the 32-bit path compute every element, as one chain of fmaf: infinities and NaN come out as they do there.
+// A sum that is not finite (an operand was infinite, NaN or above 2^104, or the sums above 2^80) is computed again as the
+// other kernels of the 32-bit path compute every element, as one chain of fmaf: infinities and NaN come out as they do there.
 //
 // Takes whole boxes only: N a multiple of 32, K of 32, rows on 16 bytes.  Every wait is bounded (status word).
 #include <cstdint>
@@ -110,13 +110,30 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Two neighbouring values as three pairs of bfloat16, the first of a pair in the low half.  All four subtractions are exact.
+// Two neighbouring values, times 2^24, as three pairs of bfloat16, the first of a pair in the low half.  All four subtractions
+// are exact, and with the factor every float32 below 2^104 is the sum of its parts: without it the last part of a value below
+// 2^-110 fell under bfloat16's smallest number (operands of 1e-35 gave products 5e-6 off, 2e-38 3e-3).  A larger value, or a sum
+// of 2^80 and more, overflows, and the element is made as one chain of fmaf.
+constexpr float SPLIT_SCALE = 16777216.f, SUM_SCALE = 1.f / (16777216.f * 16777216.f);
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  auto pair = [](float a, float b) { const __nv_bfloat162 h = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const uint32_t*>(&h); };
-  hi = pair(x, y);
-  const float rx = x - __uint_as_float(hi << 16), ry = y - __uint_as_float(hi & 0xffff0000u);
-  mid = pair(rx, ry);
-  lo = pair(rx - __uint_as_float(mid << 16), ry - __uint_as_float(mid & 0xffff0000u));
+  auto join = [](float a, float b) { uint64_t v; asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); return v; };
+  auto round = [](uint64_t v) {
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  };
+  auto less = [&](uint64_t v, uint32_t part) {      // v - part
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(join(__uint_as_float(part << 16), __uint_as_float(part & 0xffff0000u))), "l"(join(-1.f, -1.f)), "l"(v));
+    return r;
+  };
+  uint64_t v;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(join(x, y)), "l"(join(SPLIT_SCALE, SPLIT_SCALE)));
+  hi = round(v);
+  v = less(v, hi);
+  mid = round(v);
+  lo = round(less(v, mid));
 }
 
 // One element as the other kernels of the 32-bit path make it.
@@ -413,7 +430,7 @@ linear_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     float* dst = out + (size_t)gm * ldo + gn;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      if (!isfinite(sum[e])) sum[e] = chain(a + (size_t)gm * lda, w + (size_t)(gn + e) * k, k);
+      sum[e] = isfinite(sum[e]) ? sum[e] * SUM_SCALE : chain(a + (size_t)gm * lda, w + (size_t)(gn + e) * k, k);
       if (MODE == OUT_ADD) dst[e] += sum[e];
       else dst[e] = sum[e];
     }
@@ -479,9 +496,11 @@ static int launch_shape(const float* a, const float* w, float* out, int m, int n
 // CTAs on every SM, and by what a launch takes whatever it multiplies (7.8 us for 2,048 x 2,048, whose weights take 2.6); many by
 // the tensor cores and the read-out beside them.  us, m = 1 / 8 / 64 / 509, launches in a graph, weights from memory, one chain of
 // fmaf per element: 2,560 x 2,048 7.8 / 13.4 / 55 / 144, 2,048 x 2,048 7.5 / 12.9 / 37 / 101, 11,264 x 2,048 23.1 / 27.3 / 103 /
-// 458, 2,048 x 5,632 18.6 / 33.6 / 99 / 274; here 8.2 / 8.4 / 15.5 / 62, 7.8 / 8.2 / 20.9 / 42, 21.9 / 22.3 / 48 / 162, 15.6 /
-// 16.0 / 37 / 83.  With six products and parts that are cut: 8.2 / 8.6 / 14.7 / 64, 8.1 / 8.4 / 20.6 / 43, 21.9 / 22.3 / 46 / 174,
-// 16.0 / 16.3 / 35 / 89: the two products more cost 33 to 64 rows 1 to 6 %.
+// 458, 2,048 x 5,632 18.6 / 33.6 / 99 / 274; here 8.2 / 8.5 / 15.4 / 63, 7.8 / 8.3 / 20.8 / 43, 22.1 / 22.4 / 48 / 166, 15.7 /
+// 16.3 / 36 / 86.  With six products and parts that are cut: 8.2 / 8.6 / 14.7 / 64, 8.1 / 8.4 / 20.6 / 43, 21.9 / 22.3 / 46 / 174,
+// 16.0 / 16.3 / 35 / 89: the two products more cost 33 to 64 rows 1 to 6 %.  (Without the factor of split_pair 11,264 x 2,048 took
+// 162 instead of 166 for 509 rows, few rows the same; with scalar multiplications and subtractions instead of pairs eight rows took 23.5
+// and 17.8 for the two large ones.)
 // Other forms of Shape64: weights split by two groups of warps 2 to 3 % slower, three or four stages 1 to 4 %.
 //                    BN RAW STAGES DBUF W_GROUPS T_GROUPS T_WARPS E_COLS CTAS PAIRS REGS
 using Shape16 = Shape<16, 5, 3, 2, 2, 2, 1, 16, 2>;
