@@ -45,6 +45,21 @@ def test_rows_of_every_count_are_near_64_bits_and_depend_on_no_other_row(ops, n,
     assert bool(((whole - want).abs() <= most).all())
 
 
+def test_the_order_of_the_sums_follows_from_the_weight_alone(ops, monkeypatch):
+    """Neither the switch of the bfloat16 path's slices nor the number of SMs moves a bit."""
+    g = torch.Generator(device=DEV).manual_seed(5)
+    for n, k in ((2048, 2048), (8192, 2048)):
+        a, w = torch.randn(24, k, generator=g, device=DEV), torch.randn(n, k, generator=g, device=DEV)
+        outs = []
+        for split, sms in ((True, 148), (False, 148), (True, 40), (True, 160)):
+            monkeypatch.setattr(ops, "split_k", split)
+            monkeypatch.setattr(ops, "sm_count", lambda *_, sms=sms: sms)
+            out = torch.empty(24, n, device=DEV)
+            ops.linear(a, w, out)
+            outs.append(out)
+        assert all(torch.equal(o, outs[0]) for o in outs)
+
+
 def test_a_single_product_is_as_near_as_one_rounding(ops):
     """Rows of one value each: eight partial products leave 2^-34 out, and the sum is rounded once (2^-24).  With parts that are cut
     instead of rounded the first pair is 4.7e-7 off."""

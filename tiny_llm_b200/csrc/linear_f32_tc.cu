@@ -12,7 +12,7 @@
 // 1.8, 1.4, 1.3e-8 in one slice of K, 2.6e-8, 3.0, 2.9, 2.5, 1.9e-8 in eight (a rounding more per slice), the chain 2.5e-8, 2.6,
 // 2.7, 2.7, 2.9e-8.
 //
-// The sums' order is a function of N and K alone -- k ascending in blocks of 64 within each of `slices` runs of blocks, the
+// The sums' order is a function of N and K alone (`slices` must be one) -- k ascending in blocks of 64 within each of `slices` runs of blocks, the
 // runs added in pairs, pairs of pairs and so on -- whatever M is and whichever shape of the kernel takes it, so a row's
 // result does not depend on its batch, to the bit.
 //

@@ -1359,6 +1359,20 @@ def _f32_tc_ok(a: torch.Tensor, w: torch.Tensor) -> bool:
             n * k >= 1 << 20 and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def _f32_tc_slices(n: int, k: int) -> int:
+    """Slices of K of a 32-bit product on the tensor cores: 1, 2, 4 or 8, the most that make at most 296 CTAs of 128 weight rows
+    and leave four blocks of 64 to each.  The order of the sums follows from it, so it looks at the weight's sizes alone: at no
+    number of rows, switch or part (296 is two per SM of the part this was measured on).  us, one row / 8 / 131 / 512, two
+    slices and four: 8,192 x 2,048 21.1 and 15.3 / 21.5 and 15.6 / 64 and 66 / 129 and 133; four and eight: 4,096 x 2,048
+    12.7 and 10.3 / 13.1 and 10.5 / 34 and 43 / 68 and 85, 4,096 x 4,096 21.0 and 15.4 / 21.4 and 15.7 / 57 and 66 / 114 and 132 (one
+    chain of fmaf 15.1 / 25.9 / 202 / 376: one row would be the one to lose); more CTAs than that lose everywhere: 6,144 x 2,048 four
+    and eight 13.7 and 16.5 / 14.5 and 16.8 / 65 and 63 / 101 and 127."""
+    tiles, blocks, s = -(-n // 128), -(-k // 64), 1
+    while s < 8 and 2 * s * tiles <= 296 and 2 * s * 4 <= blocks:
+        s *= 2
+    return s
+
+
 def prefers_split(a: torch.Tensor, w: torch.Tensor) -> bool:
     """True when `linear` would cut K into slices for this product if it may add into a float32
     output: few rows (decode), so few weight tiles that the SMs only fill when K is split too.
@@ -1415,7 +1429,7 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool
     if _f32_tc_ok(a, w):
         lib = build.load_library("linear_f32_tc")
         _call(lib, lib.tllm_linear_f32_tc, _ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0), out.stride(0),
-                                           OUT_ACC if mode == OUT_ACC else OUT_F32, _cluster_slices(n, k), _ptr(status_word(a.device)), _stream())
+                                           OUT_ACC if mode == OUT_ACC else OUT_F32, _f32_tc_slices(n, k), _ptr(status_word(a.device)), _stream())
         return
     lib = build.load_library("linear_generic")
     _call(lib, lib.tllm_linear_generic, _ptr(a), _ptr(w), _ptr(out), m, n, k, a.stride(0), out.stride(0),
