@@ -154,3 +154,23 @@ def test_operands_that_are_not_finite_give_what_one_chain_of_fmaf_gives(ops, mon
         assert torch.equal(got[odd].nan_to_num(nan=1.5), want[odd].nan_to_num(nan=1.5))
         size = a[:m].nan_to_num(0, 0, 0).abs().double() @ w.nan_to_num(0, 0, 0).abs().double().T
         assert bool(((got.double() - want.double()).abs()[~odd] <= (size * k * 2.0 ** -23 + 1e-37)[~odd]).all())
+
+
+@pytest.mark.parametrize("m", [8, 300])
+def test_rows_of_nan_take_no_longer_than_others(ops, m):
+    """(A chain of 2,048 fmaf per element, one thread each, took many times the product.)"""
+    g = torch.Generator(device=DEV).manual_seed(m)
+    a, w, took = torch.randn(m, 2048, generator=g, device=DEV), torch.randn(11264, 2048, generator=g, device=DEV), {}
+    out = torch.empty(m, 11264, device=DEV)
+    for kind, rows in (("finite", a), ("nan", torch.full_like(a, math.nan))):
+        times = []
+        for _ in range(6):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            for _ in range(4):
+                ops.linear(rows, w, out)
+            end.record()
+            torch.cuda.synchronize()
+            times.append(begin.elapsed_time(end))
+        took[kind] = min(times)
+    assert bool(out.isnan().all()) and took["nan"] < 1.5 * took["finite"], took
