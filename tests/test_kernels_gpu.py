@@ -17,6 +17,16 @@ def tol(dtype, scale=1.0):
     return (2e-5 if dtype == "float32" else 2.0 ** -7) * scale
 
 
+def launched(ops, call):
+    """The compiled functions that a call launched, by name."""
+    ops.begin_tape()
+    try:
+        call()
+    finally:
+        tape = ops.end_tape()
+    return [fn.__name__ for _, fn, _ in tape]
+
+
 @pytest.fixture(scope="module")
 def ops():
     from tiny_llm_b200 import ops
@@ -89,7 +99,8 @@ def test_float32_linear_of_few_rows_gives_the_bits_of_the_tile_kernel(ops, m, n,
     """Up to 16 float32 rows run on a kernel of their own, products of at least 128 x 128 on 128 x 128 tiles; every
     output element is the same chain of fmaf over ascending k as in the 64 x 64 tiles, so all agree to the bit, for
     every row count, for widths and depths that fill no tile or chunk, for a strided input and when adding into the
-    output."""
+    output.  (Large weights off the tensor cores, which sum in another order.)"""
+    monkeypatch.setattr(ops, "linear_f32_tc", False)
     torch.manual_seed(m * 1000 + n)
     a = torch.randn(m, k + 8, device=DEV)[:, :k]
     w = torch.randn(n, k, device=DEV)
@@ -98,7 +109,7 @@ def test_float32_linear_of_few_rows_gives_the_bits_of_the_tile_kernel(ops, m, n,
     for skinny in (True, False):
         monkeypatch.setattr(ops, "linear_skinny", skinny)
         out = torch.empty(m, n + 4, device=DEV)[:, :n]
-        ops.linear(a, w, out)
+        assert launched(ops, lambda: ops.linear(a, w, out)) == ["tllm_linear_generic"]
         acc = torch.full((m, n), 0.25, device=DEV)
         ops.linear(a, w, acc, accumulate=True)
         outs.append((out.clone(), acc))
@@ -326,9 +337,10 @@ def test_float32_tiles_of_every_size_give_the_bits_of_the_tile_kernel(ops, m, n,
     assert float((outs[0][0][:, :n] - ref).abs().max()) <= k * 2.0 ** -23 * float(a.abs().max() * w.abs().max()) * math.sqrt(k)
 
 
-@pytest.mark.parametrize("m,n,k", [(17, 64, 64), (100, 192, 256), (509, 40, 1024)])
+@pytest.mark.parametrize("m,n,k", [(17, 64, 64), (100, 192, 256), (509, 40, 1024), (40, 512, 2048), (130, 1024, 2048)])
 def test_float32_products_of_many_rows_wait_for_weights_that_are_being_written(ops, m, n, k):
-    """`w` is the product of the launch just before, which takes long on a few SMs: the others are free for this one."""
+    """`w` is the product of the launch just before, which takes long on a few SMs: the others are free for this one.  (The last
+    two run on the tensor cores.)"""
     g = torch.Generator().manual_seed(m)
     deep = 16384
     left, right = torch.randn(n, deep, generator=g).to(DEV), (torch.randn(k, deep, generator=g) * deep ** -0.5).to(DEV)
@@ -337,7 +349,7 @@ def test_float32_products_of_many_rows_wait_for_weights_that_are_being_written(o
     ops.linear(left, right, want_w)
     want = torch.empty(m, n, device=DEV)
     torch.cuda.synchronize()
-    ops.linear(a, want_w, want)
+    assert launched(ops, lambda: ops.linear(a, want_w, want)) == ["tllm_linear_f32_tc" if k == 2048 else "tllm_linear_generic"]
     for _ in range(3):
         w, out = torch.full((n, k), math.nan, device=DEV), torch.empty(m, n, device=DEV)
         torch.cuda.synchronize()
