@@ -1,5 +1,6 @@
 """Attention of decoded tokens by TMA: slices from one to eight, tiles that end inside a page, pages of every size, requests
-of one key, several new tokens per request, slices that are empty, pages that hold NaN where no key is."""
+of one key, several new tokens per request, slices that are empty, pages that hold NaN where no key is; pages larger than a tile
+stay on the kernel that gathers."""
 import math
 import types
 
@@ -7,14 +8,15 @@ import pytest
 import torch
 
 import plain_llama as pl
-from test_kernels_gpu import paged_setup, tol
+from test_kernels_gpu import launched, paged_setup, tol
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("hd,nq,nkv,q_len,page", [(64, 32, 4, 1, 16), (64, 16, 1, 1, 64), (64, 6, 2, 5, 8), (64, 3, 3, 16, 32),
-                                                  (128, 32, 8, 1, 16), (128, 7, 1, 2, 8), (128, 4, 4, 1, 32)])
+                                                  (128, 32, 8, 1, 16), (128, 7, 1, 2, 8), (128, 4, 4, 1, 32),
+                                                  (128, 4, 4, 1, 64)])
 @pytest.mark.parametrize("slices", [1, 2, 5, 8])
 @pytest.mark.parametrize("few", [True, False])
 def test_decoded_tokens_in_slices_of_keys(hd, nq, nkv, q_len, page, slices, few, monkeypatch):
@@ -33,9 +35,10 @@ def test_decoded_tokens_in_slices_of_keys(hd, nq, nkv, q_len, page, slices, few,
         cu_q=torch.arange(0, t + 1, q_len, dtype=torch.int32).to(DEV),
         q_start=torch.tensor([l - q_len for l in lens], dtype=torch.int32).to(DEV), num_requests=n, max_q_len=q_len, max_kv_len=max(lens))
     out = torch.full((t, nq * hd), math.nan, dtype=torch.bfloat16, device=DEV)
-    ops.paged_attention(qkv.to(DEV), nq, nkv, hd, kc.to(DEV), vc.to(DEV), table.to(DEV), batch, out, hd ** -0.5, None, Workspace(DEV))
+    names = launched(ops, lambda: ops.paged_attention(qkv.to(DEV), nq, nkv, hd, kc.to(DEV), vc.to(DEV), table.to(DEV), batch, out,
+                                                      hd ** -0.5, None, Workspace(DEV)))
     ops.check_status()
-    assert f"attention_decode_head_dim{hd}" in ops.build.loaded_libraries()
+    assert names == ["tllm_attention_decode" if page * hd <= 4096 else "tllm_attention_mma"]
     out = out.float().cpu()
     for r, l in enumerate(lens):
         q = qkv[r * q_len: (r + 1) * q_len, : nq * hd].float().view(q_len, nq, hd)

@@ -7,6 +7,8 @@ import types
 import pytest
 import torch
 
+from test_kernels_gpu import launched
+
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 KD, VD = 256, 192
@@ -39,8 +41,9 @@ def test_portions_with_latent_keys(nq, nkv, page, sink):
         max_q_len=max(q_lens), max_kv_len=max(lens))
     extra = torch.randn(nq, generator=g) * 2 if sink else None
     out = torch.full((t, nq * VD), math.nan, dtype=torch.bfloat16, device=DEV)
-    ops.paged_attention_maps(q.to(DEV)[:, :nq * KD], nq, nkv, 1, KD, VD, kc.to(DEV), vc.to(DEV), table.to(DEV), batch, out, KD ** -0.5,
-                             sink=None if extra is None else extra.to(DEV), workspace=Workspace(DEV))
+    assert launched(ops, lambda: ops.paged_attention_maps(
+        q.to(DEV)[:, :nq * KD], nq, nkv, 1, KD, VD, kc.to(DEV), vc.to(DEV), table.to(DEV), batch, out, KD ** -0.5,
+        sink=None if extra is None else extra.to(DEV), workspace=Workspace(DEV))) == ["tllm_attention_maps_mma"]
     ops.check_status()
     out, group = out.double().cpu().view(t, nq, VD), nq // nkv
     for r, (n, m) in enumerate(zip(lens, q_lens)):

@@ -508,7 +508,7 @@ def _lens64():
     return [2048, 2047, 1, 64, 65] + torch.randint(1, 2049, (59,), generator=g).tolist()
 
 
-@pytest.mark.parametrize("wide", [False, True, "cluster"])
+@pytest.mark.parametrize("wide", [False, True, "cluster", "tma"])
 @pytest.mark.parametrize("bucket", [False, True])
 @pytest.mark.parametrize("hd,nq,nkv,q_len,lens,window,page", [
     (64, 32, 4, 1, [2048], None, 16),          # batch 1 at the longest context: the most key slices
@@ -526,8 +526,9 @@ def test_decode_attention_over_long_contexts(ops, hd, nq, nkv, q_len, lens, wind
     the power-of-two bucket of the longest context, as a replayed graph does, so that short requests
     have empty slices; `wide` takes the kernel with one warp per tile wherever the head size lets it (else the
     kernel that walks a slice tile by tile), "cluster" with its slices merged inside a thread-block cluster instead
-    of by a kernel behind it.  Unwritten slots of the pages are NaN; one key far back carries a query."""
+    of by a kernel behind it, "tma" the kernel that takes its tiles by TMA wherever its rule lets it.  Unwritten slots of the pages are NaN; one key far back carries a query."""
     from tiny_llm_b200.engine import Workspace
+    monkeypatch.setattr(ops, "attention_decode_tma", wide == "tma")
     monkeypatch.setattr(ops, "decode_wide_ctas", (1, 1 << 30) if wide else (1, 0))
     monkeypatch.setattr(ops, "_cluster_merge", lambda n_req, n_kv, splits: wide == "cluster" and 2 <= splits <= 8)   # at every batch
     dtype = "bfloat16"
@@ -561,8 +562,9 @@ def test_decode_attention_over_long_contexts(ops, hd, nq, nkv, q_len, lens, wind
     assert splits > 1 or max(lens) < 128
     out = torch.full((t, nq * hd), float("nan"), dtype=DT[dtype], device=DEV)
     scale = 1.0 / math.sqrt(hd)
-    ops.paged_attention(qkv.to(DEV), nq, nkv, hd, k_cache.to(DEV), v_cache.to(DEV), table.to(DEV), batch, out,
-                        scale, window, Workspace(DEV))
+    tma = wide == "tma" and window is None and ops._decode_slices(n_req, nkv, hd, max_kv) is not None
+    assert launched(ops, lambda: ops.paged_attention(qkv.to(DEV), nq, nkv, hd, k_cache.to(DEV), v_cache.to(DEV), table.to(DEV), batch, out,
+                                                     scale, window, Workspace(DEV))) == ["tllm_attention_decode" if tma else "tllm_attention_mma"]
     out = out.float().cpu()
     assert not torch.isnan(out).any()
     for r, l in enumerate(lens):
