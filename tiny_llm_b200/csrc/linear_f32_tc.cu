@@ -471,8 +471,8 @@ static int launch_mode(const float* a, const float* w, float* out, int m, int n,
   const int blocks = (k + 2 * KS - 1) / (2 * KS), per = (blocks + slices - 1) / slices;
   const int tiles_m = (m + S::BN - 1) / S::BN, tiles_n = (n + ROWS - 1) / ROWS;
   // Two slices per CTA where one each are more CTAs than SMs: what a CTA pays once, its first steps' way from memory and its
-  // sums' way out, comes half as often.  (us, eight CTAs of one slice / four of two: 509 rows, 2,560 x 2,048 92 / 66, 2,048 x
-  // 2,048 76 / 45, 2,048 x 5,632 135 / 93; 131 rows, 2,048 x 2,048 39 / 23.)
+  // sums' way out, comes half as often.  (us, eight CTAs of one slice / four of two: 509 rows, 2,560 x 2,048 92 / 63, 2,048 x
+  // 2,048 76 / 43, 2,048 x 5,632 130 / 86; 131 rows, 2,048 x 2,048 39 / 21.)
   const int each = S::PAIRS && slices > 2 && (long long)tiles_m * tiles_n * slices > sms ? 2 : 1, ctas = (slices + each - 1) / each;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles_m, tiles_n, ctas);

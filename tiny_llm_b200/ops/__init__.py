@@ -1344,11 +1344,16 @@ def fused_qkv_preferred(m: int, n: int, k: int) -> bool:
 linear_skinny = True
 
 
-# float32 products of large weights on the tensor cores, every factor as three bfloat16 parts that add up to it exactly
+# float32 products of large weights on the tensor cores, every factor as three bfloat16 parts that add up to it
 # (csrc/linear_f32_tc.cu): whole boxes, rows of at least 2,048 values, at least 2^20 weights.  The rule may not look at the
-# number of rows, since the kernels' sums have other bits.  us, one chain of fmaf / this: 512 x 2,048 one row 7.9 / 7.2, 16
-# 12.7 / 7.6, 100 38 / 15; 256 x 4,096 13.9 / 10.0, 23.5 / 10.4, 72 / 21; with shorter rows few rows of A lose more than many
-# gain: 1,024 x 1,024 4.8 / 7.3, 8.0 / 7.6, 20 / 14; 2,048 x 512 3.4 / 7.4, 6.2 / 7.5, 16 / 14.
+# number of rows, since the kernels' sums have other bits, so the line lies where one row, which one chain of fmaf serves
+# best, stops losing more than a quarter.  us, one chain of fmaf / this, for one row, 8, 16, 64 and 512 of A:
+#   K = 1,024, 1,024 weight rows 4.3 / 6.5, 6.5 / 6.7, 7.3 / 6.9, 19 / 10, 37 / 15; 8,192 7.1 / 10.2, 13.9 / 10.6, 23 / 11, 36 / 16, 187 / 86
+#   K = 1,536, 1,024             5.8 / 8.2, 8.9 / 8.3, 11.0 / 8.5, 28 / 12, 54 / 18; 8,192 9.8 / 12.5, 20 / 13, 33 / 13, 54 / 21, 278 / 111
+#   K = 2,048, 1,024             7.3 / 6.7, 11.7 / 7.0, 14.8 / 7.3, 37 / 11, 71 / 22; 8,192 12.2 / 15.3, 26 / 16, 43 / 16, 71 / 25, 367 / 135
+#   K = 2,048, 512 (2^20 weights) 7.3 / 6.5, 10.4 / 6.7, 12.2 / 7.0, 37 / 10, 55 / 30
+# Left out though faster at every number of rows: 32,000 weight rows of K = 512 to 1,536 (16.4 / 15.0 and 26 / 25 and 36 / 34 for one
+# row, 50 / 32 to 143 / 67 for 64) and 256 of K = 2,048 (7.3 / 6.3, 37 / 11).
 # TLLM_LINEAR_F32_TC=0 turns it off.
 linear_f32_tc = os.environ.get("TLLM_LINEAR_F32_TC", "1") != "0"
 
@@ -1387,8 +1392,8 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool
     accumulate=True adds the product into a float32 `out`.  cluster_slices=True: a product of at most 128 rows
     that stores bfloat16 cuts K into slices that meet in a thread-block cluster (every SM streams weights; without
     it such a product has one CTA per 128 output columns, which walks all of K).  bfloat16 products run on the tensor
-    cores (tcgen05) when K and the row stride of `a` are multiples of 8; large float32 products run there as sums of exact
-    parts (_f32_tc_ok); other float32 products, and the sizes TMA cannot take, run on the SIMT kernel.
+    cores (tcgen05) when K and the row stride of `a` are multiples of 8; large float32 products run there as sums of
+    bfloat16 parts that keep 32 bits (_f32_tc_ok); other float32 products, and the sizes TMA cannot take, run on the SIMT kernel.
     `w` is taken for a loaded weight: float32 products of at most 16 rows and the tensor-core products begin to read it
     while earlier launches of this package still run, so none of those may be writing it.  (float32 products of more
     rows wait first.)"""
@@ -1509,9 +1514,10 @@ def _attention_splits(num_requests: int, max_q_len: int, group: int, num_kv_head
     return max(1, min(-(-2 * sms // ctas), max_kv_len // 256))
 
 
-# Decoded tokens with one warp per 64-key tile (slices of four tiles, all of a slice's copies in flight at once, one
-# block barrier instead of one per tile): taken when it gives this many CTAs.  Measured at the TinyLlama sizes,
-# context 2,048, against the kernel that walks a slice tile by tile with four warps per tile (ms per step): batch 4
+# Decoded tokens that the kernel by TMA (below) leaves to the ones that gather: windows, other head sizes, pages under 8 keys or
+# over a tile, one or two requests over long contexts.  One warp per 64-key tile (slices of four tiles, all of a slice's copies
+# in flight at once, one block barrier instead of one per tile): taken when it gives this many CTAs.  Measured at the TinyLlama
+# sizes, context 2,048, before the kernel by TMA took them, against the kernel that walks a slice tile by tile with four warps per tile (ms per step): batch 4
 # 0.754 / 0.778, 8 0.810 / 0.826, 16 0.938 / 0.942; outside the range it loses: batch 1 0.724 / 0.716 (32 CTAs),
 # batch 32 1.193 / 1.124 (1,024 CTAs).  TLLM_DECODE_WIDE=0 turns it off (a switch for measurements).
 decode_wide_ctas = (96, 640) if os.environ.get("TLLM_DECODE_WIDE", "1") != "0" else (1, 0)
@@ -1543,10 +1549,11 @@ def _wide_splits(num_requests: int, num_kv_heads: int, max_kv_len: int) -> int:
 # Decoded tokens of head size 64 or 128 without a window, pages of at most a tile: the kernel that fetches its tiles by TMA
 # (csrc/attention_decode.cu), in slices of at most eight tiles by smaller CTAs, three to an SM, else by larger ones, two to an
 # SM; as many slices (up to the 8 of a portable cluster) as one wave of CTAs holds, one tile per warp at least.  us per launch,
-# this kernel / the ones above: 4 key rows of 64, 64 requests with 300, 700, 1,400 keys 6.9 / 11.7, 9.9 / 17.4, 15.9 / 23.7,
-# 16 with 1,400 7.7 / 11.6, 8 with 1,400 6.4 / 6.5, 1 with 300 4.6 / 5.2; 8 key rows of 128, 16 requests with 1,400 and
-# 5,600 18.6 / 25.4, 56.0 / 71.7.  Not where eight slices leave SMs idle and are long, which the merge by a kernel of its own
-# can cut finer: 8 x 128, 5,600 keys, one request 15.9 / 12.6, two 17.3 / 15.3, four (256 CTAs) 19.0 / 27.5.
+# this kernel / the ones above, launches in a graph, caches from memory: 4 key rows of 64, 64 requests with 300, 700, 1,400 keys
+# 7.0 / 11.3, 10.3 / 14.2, 17.2 / 27.1, 16 with 1,400 7.9 / 11.2, 8 with 1,400 5.8 / 6.4, 1 with 300 4.3 / 4.7; 8 key rows of 128,
+# 16 requests with 1,400 and 5,600 19.5 / 20.1, 60.3 / 74.4, four with 5,600 (256 CTAs) 19.6 / 20.9.  Not where eight slices leave
+# SMs idle and are long, which the merge by a kernel of its own can cut finer: 8 x 128, 5,600 keys, one request 15.9 / 12.6, two
+# 17.3 / 15.3 (by themselves).
 # TLLM_ATTENTION_DECODE_TMA=0 turns it off (a switch for measurements).
 attention_decode_tma = os.environ.get("TLLM_ATTENTION_DECODE_TMA", "1") != "0"
 
